@@ -207,9 +207,9 @@ int ensure_workspace(tsdfl_ctx* c, size_t P, size_t N)
     return TSDFL_OK;
 }
 
-int ensure_resample_ws(tsdfl_ctx* c, size_t M)
+// need: resample_workspace_bytes(M) or residual_workspace_bytes(M).
+int ensure_resample_ws(tsdfl_ctx* c, size_t need)
 {
-    size_t need = resample_workspace_bytes(M);
     if (need <= c->rs_bytes) return TSDFL_OK;
     need = std::max(need, c->rs_bytes + c->rs_bytes / 4);
     void* p = nullptr;
@@ -848,7 +848,7 @@ int tsdfl_ctx_reserve(tsdfl_ctx* c, size_t P, size_t N)
     if (rc) return rc;
     rc = ensure_workspace(c, P, N);
     if (rc) return rc;
-    return ensure_resample_ws(c, P);
+    return ensure_resample_ws(c, std::max(resample_workspace_bytes(P), residual_workspace_bytes(P)));
 }
 
 int tsdfl_map_create(tsdfl_ctx* ctx, const tsdfl_map_coef* coef, const int32_t* grid_occ, const float* data,
@@ -1130,7 +1130,7 @@ int resample_systematic_host(tsdfl_ctx* c, const char* fn, const float* src, siz
     }
     int rc = set_device(c->device);
     if (rc) return rc;
-    rc = ensure_resample_ws(c, M);
+    rc = ensure_resample_ws(c, resample_workspace_bytes(M));
     if (rc) return rc;
     size_t w_b = align_up(sizeof(float) * stride * M, 256);
     size_t i_b = align_up(sizeof(uint32_t) * (cap ? cap : 1), 256);
@@ -1179,7 +1179,7 @@ int tsdfl_resample_systematic_device(tsdfl_ctx* c, const float* d_particles, siz
     }
     int rc = set_device(c->device);
     if (rc) return rc;
-    rc = ensure_resample_ws(c, M);
+    rc = ensure_resample_ws(c, resample_workspace_bytes(M));
     if (rc) return rc;
     return launch_resample_impl(d_particles, d_particles + 6, 7, M, u0, d_particles_out, nullptr, cap, d_count,
                                 c->rs_ws, c->status, c->stream);
@@ -1200,7 +1200,7 @@ int tsdfl_resample_residual_systematic(tsdfl_ctx* c, const float* weights, size_
     }
     int rc = set_device(c->device);
     if (rc) return rc;
-    rc = ensure_resample_ws(c, M);
+    rc = ensure_resample_ws(c, residual_workspace_bytes(M));
     if (rc) return rc;
     size_t w_b = align_up(sizeof(float) * M, 256);
     size_t i_b = align_up(sizeof(uint32_t) * (cap ? cap : 1), 256);
@@ -1237,7 +1237,7 @@ int tsdfl_resample_residual_systematic_device(tsdfl_ctx* c, const float* d_parti
     }
     int rc = set_device(c->device);
     if (rc) return rc;
-    rc = ensure_resample_ws(c, M);
+    rc = ensure_resample_ws(c, residual_workspace_bytes(M));
     if (rc) return rc;
     return launch_resample_residual(d_particles, d_particles + 6, 7, M, u0, d_particles_out, nullptr, cap, d_count,
                                     c->rs_ws, c->status, c->stream);

@@ -1,0 +1,47 @@
+// Programmatic dependent launch for the kernels that follow one another in a
+// stream (the update and resampling chains, the scan reduction).
+#pragma once
+
+#include <cuda_runtime.h>
+
+namespace tsdfl {
+
+// First statement of every kernel that launch_chained starts with programmatic
+// dependent launch: the grid may be scheduled while the previous kernel in the
+// stream is still running, so it waits here until that kernel has completed and
+// its writes are visible, then lets its own successor be scheduled once all of
+// its CTAs have started (the successor waits in turn).  Both instructions do
+// nothing for a grid launched without the attribute.
+static __device__ __forceinline__ void chain_enter()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Launches a kernel that opens with chain_enter(), so that its launch overlaps
+// the end of the previous kernel instead of following it.
+template <typename... Params, typename... Args>
+inline void launch_chained_2d(void (*kernel)(Params...), dim3 grid, unsigned block, size_t smem, cudaStream_t s,
+                              Args... args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+template <typename... Params, typename... Args>
+inline void launch_chained(void (*kernel)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
+                           Args... args)
+{
+    launch_chained_2d(kernel, dim3(grid), block, smem, s, args...);
+}
+
+}  // namespace tsdfl

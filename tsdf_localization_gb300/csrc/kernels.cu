@@ -8,6 +8,7 @@
 #include <atomic>
 #include <vector>
 
+#include "chain.h"
 #include "index_math.h"
 #include "subsample.h"
 #include "tsdfl_internal.h"
@@ -102,19 +103,6 @@ __device__ __forceinline__ uint32_t warp_sum_u32(uint32_t v)
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
-}
-
-// First statement of every kernel of the update and resampling chain, which
-// the launchers start with programmatic dependent launch: the grid may be
-// scheduled while the previous kernel in the stream is still running, so it
-// waits here until that kernel has completed and its writes are visible, then
-// lets its own successor be scheduled once all of its CTAs have started (the
-// successor waits in turn).  Both instructions do nothing for a grid launched
-// without the attribute.
-__device__ __forceinline__ void chain_enter()
-{
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // Element-wise min (x, y) / max (z, w) over the warp; NaN entries are ignored.
@@ -1884,7 +1872,6 @@ __global__ void resample_assign_kernel(const float* particles, int M, float* out
 }
 
 constexpr int kChainTile = 2048;
-constexpr int kChainThreads = 512;
 
 // Fallback of the parallel systematic path for weights that are not exact
 // multiples of 2^-52 (tiny or huge) but non-negative and finite: the serial
@@ -2400,111 +2387,6 @@ __device__ void systematic_chain_block(const float* __restrict__ w, int stride, 
     }
 }
 
-// ResidualSystematicResampler::resample (novel_resampling.h:76-104) for
-// weights w >= 0 with (float)M * w < 2^22 - 1 (others stop it with *err): one
-// thread walks the draw chain -- temp = (float)M w - u; o = floor(temp) + 1,
-// the reference's (size_t)(temp + 1.0); u = (float)o - temp -- over tiles of
-// (float)M w staged in shared memory, four dependent float additions a
-// particle and nothing else; the block then turns the counts into offsets with
-// a scan.
-__global__ void __launch_bounds__(kChainThreads) residual_chain_kernel(const float* __restrict__ w, int stride,
-                                                                       int M, float u0, uint32_t* __restrict__ cnt,
-                                                                       uint32_t* __restrict__ off,
-                                                                       unsigned long long* total, int* err)
-{
-    static_assert(kChainTile == 4 * kChainThreads, "four counts per thread in the scan");
-    __shared__ float sc[kChainTile];   // (float)M * w, then the counts
-    __shared__ uint32_t warp_tot[kChainThreads / 32];
-    __shared__ uint32_t s_base;
-    const float Mf = (float)M;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float u = u0;
-    if (threadIdx.x == 0) s_base = 0u;
-    for (int base = 0; base < M; base += kChainTile) {
-        const int t = min(kChainTile, M - base);
-        bool bad = false;
-        for (int i = threadIdx.x; i < t; i += blockDim.x) {
-            const float x = w[(size_t)(base + i) * stride];
-            const float c = __fmul_rn(Mf, x);
-            bad |= !(x >= 0.0f) || !(c < 4194303.0f);
-            sc[i] = c;
-        }
-        if (__syncthreads_or(bad ? 1 : 0)) {
-            if (threadIdx.x == 0) {
-                *err = 1;
-                *total = s_base;
-            }
-            return;
-        }
-        if (threadIdx.x == 0) {
-            // 32 products to registers at a time, so that only the chain is serial
-            int i = 0;
-            for (; i + 32 <= t; i += 32) {
-                float v[32];
-#pragma unroll
-                for (int k = 0; k < 32; ++k) v[k] = sc[i + k];
-#pragma unroll
-                for (int k = 0; k < 32; ++k) {
-                    const float temp = __fsub_rn(v[k], u);
-                    // floor(temp) + 1 for -1 <= temp < 2^22: rounding temp + 1.5 * 2^23 down
-                    // lands on an integer (unit spacing there), so both steps are exact
-                    const float of = __fsub_rn(__fadd_rd(temp, 12582912.0f), 12582911.0f);
-                    u = __fsub_rn(of, temp);
-                    v[k] = of;
-                }
-#pragma unroll
-                for (int k = 0; k < 32; ++k) sc[i + k] = v[k];
-            }
-            for (; i < t; ++i) {
-                const float temp = __fsub_rn(sc[i], u);
-                const float of = __fsub_rn(__fadd_rd(temp, 12582912.0f), 12582911.0f);
-                u = __fsub_rn(of, temp);
-                sc[i] = of;
-            }
-        }
-        __syncthreads();
-        // exclusive offsets of this tile's counts, four per thread
-        uint32_t v[4], run = 0;
-        for (int k = 0; k < 4; ++k) {
-            const int i = 4 * threadIdx.x + k;
-            v[k] = i < t ? (uint32_t)sc[i] : 0u;
-            run += v[k];
-        }
-        uint32_t x = run;
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        if (lane == 31) warp_tot[warp] = x;
-        __syncthreads();
-        uint32_t woff = 0, tile_total = 0;
-        for (int k = 0; k < kChainThreads / 32; ++k) {
-            if (k < warp) woff += warp_tot[k];
-            tile_total += warp_tot[k];
-        }
-        uint32_t o = s_base + woff + x - run;
-        for (int k = 0; k < 4; ++k) {
-            const int i = 4 * threadIdx.x + k;
-            if (i < t) {
-                cnt[base + i] = v[k];
-                off[base + i] = o;
-            }
-            o += v[k];
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            s_base += tile_total;
-            if (s_base >= (1u << 31)) *err = 1;   // offsets stay 32-bit
-        }
-        __syncthreads();
-        if (*err) {
-            if (threadIdx.x == 0) *total = s_base;
-            return;
-        }
-    }
-    if (threadIdx.x == 0) *total = s_base;
-}
-
 // Copies particle m (7 floats) to its cnt[m] output slots below cap, or writes
 // its index there; thread 0 reports the count (and the chain's failure).
 __device__ void scatter_block(const float* particles, int M, const uint32_t* cnt, const uint32_t* off,
@@ -2534,15 +2416,6 @@ __device__ void scatter_block(const float* particles, int M, const uint32_t* cnt
         }
     }
 }
-
-__global__ void resample_scatter_kernel(const float* particles, int M, const uint32_t* cnt, const uint32_t* off,
-                                        const unsigned long long* total, const int* err, float* out,
-                                        uint32_t* idx_out, long long cap, uint32_t* count_out, int32_t* status)
-{
-    scatter_block(particles, M, cnt, off, total, err, out, idx_out, cap, count_out, status);
-}
-
-__global__ void set_int_kernel(int* p, int v) { *p = v; }
 
 // Best particle of mcl_3d.cpp:382-394: the first index with the largest weight
 // above 0 (strict comparison from max_value = 0).  Keys (weight bits, ~index)
@@ -2635,26 +2508,6 @@ int check(cudaError_t e)
 }  // namespace
 
 // ------------------------------------------------------------------ launchers
-
-// Launches a kernel of the update / resampling chain with programmatic
-// dependent launch (the kernel opens with chain_enter()), so its launch
-// overlaps the end of the previous kernel instead of following it.
-template <typename... Params, typename... Args>
-void launch_chained(void (*kernel)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
-                    Args... args)
-{
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, args...);
-}
 
 int launch_pose_prepare(const float* tf, const float* particles, int P, const float* points, int N, int npad,
                         float max_range_sq, float c_in, float c_out, const float* code_values, int shift,
@@ -3012,24 +2865,6 @@ int launch_resample_impl(const float* particles, const float* w, int stride, siz
                    (long long)cap, count_out, ws, status, (const uint32_t*)cnt, (const uint32_t*)off,
                    (const unsigned long long*)total, (const int*)err);
     g_launches += 8;
-    return check(cudaGetLastError());
-}
-
-int launch_resample_residual(const float* particles, const float* w, int stride, size_t M, float u0, float* out,
-                             uint32_t* idx_out, size_t cap, uint32_t* count_out, void* workspace, int32_t* status,
-                             cudaStream_t s)
-{
-    char* p = static_cast<char*>(workspace);
-    uint32_t* cnt = reinterpret_cast<uint32_t*>(p);
-    uint32_t* off = cnt + M;
-    unsigned long long* total = reinterpret_cast<unsigned long long*>(p + ((8 * M + 15) / 16) * 16);
-    int* err = reinterpret_cast<int*>(total + 1);
-    set_int_kernel<<<1, 1, 0, s>>>(err, 0);
-    residual_chain_kernel<<<1, kChainThreads, 0, s>>>(w, stride, (int)M, u0, cnt, off, total, err);
-    resample_scatter_kernel<<<(unsigned)((M + 255) / 256), 256, 0, s>>>(particles, (int)M, cnt, off, total, err,
-                                                                         out, idx_out, (long long)cap, count_out,
-                                                                         status);
-    g_launches += 3;
     return check(cudaGetLastError());
 }
 

@@ -278,7 +278,8 @@ size_t resample_workspace_bytes(size_t M);
 int launch_resample_impl(const float* particles, const float* w, int stride, size_t M, float u0, float* out,
                          uint32_t* idx_out, size_t cap, uint32_t* count_out, void* workspace, int32_t* status,
                          cudaStream_t s, const float* u0p = nullptr);
-// ResidualSystematicResampler on the device; workspace: resample_workspace_bytes(M).
+// ResidualSystematicResampler on the device (residual.cu); workspace: residual_workspace_bytes(M).
+size_t residual_workspace_bytes(size_t M);
 int launch_resample_residual(const float* particles, const float* w, int stride, size_t M, float u0, float* out,
                              uint32_t* idx_out, size_t cap, uint32_t* count_out, void* workspace, int32_t* status,
                              cudaStream_t s);
