@@ -145,6 +145,7 @@ size_t eval_layout(size_t nP, size_t nN, char* base, EvalBuffers* e, double** su
     size_t o_lfx = take(sizeof(long long) * kNumCodes);
     size_t o_lf = take(sizeof(float) * kNumCodes);
     size_t o_cnt = take(sizeof(int32_t) * 16);
+    size_t o_work = take(sizeof(uint32_t) * kWorkWords);
     size_t o_part = take(sizeof(double) * 256 * 10);
     size_t o_sums = take(sizeof(double) * 16);
     size_t o_wsf = take(sizeof(float) * 4);
@@ -172,6 +173,7 @@ size_t eval_layout(size_t nP, size_t nN, char* base, EvalBuffers* e, double** su
         e->lut_fx = reinterpret_cast<long long*>(b + o_lfx);
         e->lut_f = reinterpret_cast<float*>(b + o_lf);
         e->counts = reinterpret_cast<int32_t*>(b + o_cnt);
+        e->work = reinterpret_cast<uint32_t*>(b + o_work);
         e->partials = reinterpret_cast<double*>(b + o_part);
         e->sums = reinterpret_cast<double*>(b + o_sums);
         e->weight_sum_f = reinterpret_cast<float*>(b + o_wsf);
@@ -302,8 +304,8 @@ int validate_coef(const tsdfl_map_coef* c)
 // The kSentinels codes after the last slot of a code array (MapView::codes_sent).
 cudaError_t write_sentinels(uint16_t* arr, size_t at, cudaStream_t s)
 {
-    static const uint16_t kSent[kSentinels] = {(uint16_t)kCodeMiss, (uint16_t)kCodeLater, (uint16_t)kCodeNone,
-                                               (uint16_t)kCodeNone};
+    static const uint16_t kSent[kSentinels] = {(uint16_t)kCodeMiss, (uint16_t)kCodeMiss, (uint16_t)kCodeMiss,
+                                               (uint16_t)kCodeMiss};
     return cudaMemcpyAsync(arr + at, kSent, sizeof(kSent), cudaMemcpyHostToDevice, s);
 }
 
@@ -401,10 +403,9 @@ void fill_view(tsdfl_map* m)
     // within +-sub_dim^3 <= 2^21) and every sub-voxel index stays inside its
     // brick, so slot indices land in [r S^3 - S^3, r S^3 + S^3)
     const uint64_t S3 = c.sub_dim * c.sub_dim_2;
-    auto fmax_trunc = [&](int32_t mmax) { return mmax < 0 ? 0ull : (uint64_t)std::min<int64_t>(mmax, 4194303); };
-    const uint64_t up_max = fmax_trunc(v.mmax_x) + fmax_trunc(v.mmax_y) * c.up_dim_x + fmax_trunc(v.mmax_z) * c.up_dim_2;
-    v.tiled = v.sub_fast != 0 && m->codes != nullptr && m->codes_pre == S3 && S3 <= (1ull << 21) && up_max < (1ull << 23) &&
-              c.grid_occ_size < (1ull << 23) && max_sub_index(c.resolution) < c.sub_dim ? 1 : 0;
+    v.tiled = v.sub_fast != 0 && m->codes != nullptr && m->codes_pre == S3 && S3 <= (1ull << 21) &&
+              brick_reach(c) <= (1ull << 23) && c.grid_occ_size < (1ull << 23) &&
+              max_sub_index(c.resolution) < c.sub_dim ? 1 : 0;
     v.min0 = c.min_x == 0.0f && c.min_y == 0.0f && c.min_z == 0.0f && !std::signbit(c.min_x) &&
              !std::signbit(c.min_y) && !std::signbit(c.min_z) ? 1 : 0;
     v.up_dim_x_f = (float)c.up_dim_x;
@@ -415,21 +416,22 @@ void fill_view(tsdfl_map* m)
     // negative sub-voxel index (an empty range when not even layer 0 passes)
     v.zhi = v.mmax_z < 0 ? 0.0f : (float)std::min<int64_t>((int64_t)v.mmax_z + 1, 4194304);
     v.zlo = v.mmax_z < 0 ? 0.0f : -1.0f;
-    v.neg_zero = -0.0f;
+    float far[4];
+    miss_bounds(c, v.mmax_x, v.mmax_y, far);
+    v.far_limit = far[0];
+    v.far_x = far[1];
+    v.far_y = far[2];
+    v.far_z = far[3];
     const uint32_t kMag = 0x4B000000u, kMag15 = 0x4B400000u;
     v.upb_lim = kMag + (uint32_t)std::min<uint64_t>(c.grid_occ_size, 1ull << 23);
     v.sent_miss = (uint32_t)c.data_size + kMag15;
-    v.sent_later = v.sent_miss + 1u;
-    v.sent_none = v.sent_miss + 2u;
     v.codes_b = (unsigned long long)(uintptr_t)m->codes - 2ull * kMag15;
     v.grid_uxy1 = c.up_dim_2 ? (uint32_t)(c.up_dim_2 - 1) : 0u;
     v.grid_b = 0;
-    v.gsent_miss = v.gsent_later = v.gsent_none = 0;
+    v.gsent_miss = 0;
     if (m->grid) {
         v.grid_b = (unsigned long long)(uintptr_t)m->grid + 2ull * S3 - 2ull * kMag15;
         v.gsent_miss = (uint32_t)(m->grid_codes - S3) + kMag15;
-        v.gsent_later = v.gsent_miss + 1u;
-        v.gsent_none = v.gsent_miss + 2u;
     }
 }
 
@@ -446,8 +448,10 @@ int build_grid(tsdfl_map* m, cudaStream_t s)
 {
     const tsdfl_map_coef& c = m->coef;
     const uint64_t S3 = c.sub_dim * c.sub_dim_2;
+    // where coordinates past the last brick of a row alias into the next one, a
+    // lookup below the floor can reach a brick that has no skirt
     if (max_sub_index(c.resolution) >= c.sub_dim || !m->codes || m->codes_pre != S3 || c.grid_occ_size == 0 ||
-        c.grid_occ_size >= (1ull << 23))
+        c.grid_occ_size >= (1ull << 23) || brick_reach(c) > c.grid_occ_size)
         return TSDFL_OK;
     const uint64_t n = (c.grid_occ_size + c.up_dim_2) * S3;
     if (n >= (1ull << 31)) return TSDFL_OK;
@@ -471,9 +475,10 @@ int build_compact(tsdfl_map* m, const int32_t* go)
     const uint64_t gos = c.grid_occ_size;
     if (max_sub_index(c.resolution) >= c.sub_dim || !m->codes || m->codes_pre != c.sub_dim * c.sub_dim_2)
         return TSDFL_OK;   // brick table only
-    const uint64_t words = (gos + 31) / 32;
+    // zero words for every brick index a lookup inside the fast domain can form
+    const uint64_t words = (std::max(gos, brick_reach(c)) + 31) / 32;
     uint64_t bytes = 16;
-    while (bytes < 8 * words) bytes *= 2;
+    while (bytes < 8 * words && bytes <= (1u << 17)) bytes *= 2;
     if (bytes > (1u << 17)) return TSDFL_OK;
     std::vector<uint32_t> occ(bytes / 4, 0u);
     for (uint64_t up = 0; up < gos; ++up)
@@ -591,8 +596,16 @@ int map_common(tsdfl_ctx* ctx, const tsdfl_map_coef* coef, const int32_t* grid_o
     for (int k = 0; k < kNumCodes; ++k) m->max_value = std::fmax(m->max_value, std::fabs(vals[k]));
     CUDA_TRY(cudaMalloc(&m->values, sizeof(vals)));
     CUDA_TRY(cudaMemcpyAsync(m->values, vals, sizeof(vals), cudaMemcpyHostToDevice, ctx->stream));
-    size_t go = sizeof(int32_t) * (coef->grid_occ_size ? coef->grid_occ_size : 1);
+    // -1 beyond the table, up to every brick index a lookup inside the tiled
+    // kernels' fast domain can form (maps that reach further are not scored by them)
+    const uint64_t reach = brick_reach(*coef);
+    const size_t slots = std::max<uint64_t>(std::max<uint64_t>(coef->grid_occ_size, 1),
+                                            reach <= (1ull << 23) ? reach : 0);
+    size_t go = sizeof(int32_t) * slots;
     CUDA_TRY(cudaMalloc(&m->grid_occ, go));
+    if (slots > coef->grid_occ_size)
+        CUDA_TRY(cudaMemsetAsync(m->grid_occ + coef->grid_occ_size, 0xff,
+                                 sizeof(int32_t) * (slots - coef->grid_occ_size), ctx->stream));
     if (coef->grid_occ_size)
         CUDA_TRY(cudaMemcpyAsync(m->grid_occ, grid_occ, sizeof(int32_t) * coef->grid_occ_size,
                                  cudaMemcpyHostToDevice, ctx->stream));
@@ -619,13 +632,7 @@ int run_eval(tsdfl_ctx* c, const tsdfl_map* map, const tsdfl_model* mdl, float* 
     const float max_range_sq = mdl->max_range * mdl->max_range;
     const float c_in = mdl->a_range * inv_max_range;
     const float c_out = mdl->a_max;
-    // fixed-point scale: sums of N values below max_value stay below 2^62
-    int shift = 40;
-    {
-        double bound = std::fmax((double)map->max_value, 1e-30) * (double)(N + 1);
-        int need = (int)std::ceil(std::log2(bound));
-        if (62 - need < shift) shift = 62 - need;
-    }
+    const int shift = fixed_shift(map->max_value, (double)N);
     const int npad = (int)align_up(N, 4);
     cudaStream_t s = c->stream;
     rc = launch_pose_prepare(tf, d_particles, (int)P, d_points, (int)N, npad, max_range_sq, c_in, c_out, map->values,
@@ -679,12 +686,7 @@ int run_eval_sub(tsdfl_ctx* c, const tsdfl_map* map, const tsdfl_model* mdl, flo
     const float max_range_sq = mdl->max_range * mdl->max_range;
     const float c_in = mdl->a_range * inv_max_range;
     const float c_out = mdl->a_max;
-    int shift = 40;
-    {
-        double bound = std::fmax((double)map->max_value, 1e-30) * (double)(K + 1);
-        int need = (int)std::ceil(std::log2(bound));
-        if (62 - need < shift) shift = 62 - need;
-    }
+    const int shift = fixed_shift(map->max_value, (double)K);
     const int npad = (int)align_up(N, 4);
     cudaStream_t s = c->stream;
     rc = launch_pose_prepare(tf, d_particles, (int)P, d_points, (int)N, npad, max_range_sq, c_in, c_out, map->values,
@@ -1438,9 +1440,7 @@ void per_configure(tsdfl_batch::Per& q, const tsdfl_filter& F, int sm_count)
 {
     q.b.particles = F.d_particles;
     q.npad = (int)align_up(F.N, 4);
-    double bound = std::fmax((double)F.map->max_value, 1e-30) * (double)(F.N + 1);
-    int need = (int)std::ceil(std::log2(bound));
-    q.shift = 62 - need < 40 ? 62 - need : 40;
+    q.shift = fixed_shift(F.map->max_value, (double)F.N);
     const MapView& m = F.map->view;
     q.dense = F.map->occ != nullptr;
     q.tiled = m.storage == 0 && m.tiled != 0;

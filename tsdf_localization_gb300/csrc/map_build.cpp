@@ -117,6 +117,24 @@ int32_t coarse_mmax(uint64_t dim, float res)
     return 4194304;
 }
 
+uint64_t brick_reach(const tsdfl_map_coef& c)
+{
+    auto last = [&](uint64_t dim) {
+        const int32_t m = coarse_mmax(dim, c.resolution);
+        return m < 0 ? 0ull : (uint64_t)std::min<int32_t>(m, 4194303);
+    };
+    return last(c.dim_x) + last(c.dim_y) * c.up_dim_x + last(c.dim_z) * c.up_dim_2 + 1;
+}
+
+void miss_bounds(const tsdfl_map_coef& c, int32_t mmax_x, int32_t mmax_y, float far[4])
+{
+    const float open = -INFINITY;
+    far[0] = c.resolution <= 1.0f ? 4194304.0f : 0.0f;
+    far[1] = c.sub_dim % 2 == 0 ? -1.0f : open;
+    far[2] = (int64_t)mmax_x < (int64_t)c.up_dim_x ? -1.0f : open;
+    far[3] = (int64_t)mmax_x + (int64_t)mmax_y * (int64_t)c.up_dim_x < (int64_t)c.up_dim_2 ? -1.0f : open;
+}
+
 // Smallest non-negative float s (searched up to 2.0) for which pred(s) holds;
 // pred must be monotone in s.  2.0 when it never holds below 2.
 template <class Pred>

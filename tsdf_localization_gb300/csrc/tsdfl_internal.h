@@ -4,6 +4,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+#include <cmath>
+
 #include "map_host.h"
 #include "tsdfl.h"
 
@@ -14,8 +17,8 @@ namespace tsdfl {
 // the dense layout (a miss).
 constexpr int kCodeInit = 600;
 constexpr int kCodeMiss = 601;
-constexpr int kCodeNone = 602;   // no point (padding): no hit, contributes 0
-constexpr int kCodeLater = 603;  // scored later by the exact slow tiers: no hit, contributes 0 here
+constexpr int kCodeNone = 602;   // no point (padding): no hit, contributes 0 (never stored)
+constexpr int kCodeLater = 603;  // scored later by the exact slow tiers: no hit, contributes 0 here (never stored)
 constexpr int kNumCodes = 604;
 constexpr uint32_t kMissIndex = 0xffffffffu;
 
@@ -81,9 +84,9 @@ struct MapView {
     // within that bound.
     const uint2* hash;
     uint32_t hash_mask, hash_shift, hash_probes;
-    // Both code arrays end in kSentinels extra entries {kCodeMiss, kCodeLater,
-    // kCodeNone, kCodeNone}: the fast path gathers a lookup that falls outside
-    // the allocated slots from there, so every gather yields the final code.
+    // Both code arrays end in kSentinels extra codes of kCodeMiss: the fast path
+    // gathers a lookup that falls outside the allocated slots from there, so
+    // every gather yields a code.
     uint32_t codes_sent;           // index of the first sentinel in codes
     // Tiled fast path (eval_tiled_kernel, eval_batch_kernel), verified on the
     // host: brick indices below 2^23 and sub-voxel indices below sub_dim, so
@@ -96,9 +99,11 @@ struct MapView {
     int32_t min0;                  // the map's min corner is (0, 0, 0): offsets are the coordinates
     float up_dim_x_f, up_dim_2_f, sub_dim_f, sub_dim_2_f;
     float zlo, zhi;                // fast z offsets: zlo < oz < zhi
-    float neg_zero;                // -0.0f: the addend of exact products formed by FMA
+    // certain_miss (index_math.h): set by miss_bounds (map_host.h).
+    float far_limit;               // offsets it speaks about lie below this in magnitude
+    float far_x, far_y, far_z;     // offsets at or below are misses (far_y: with oz < 1)
     uint32_t upb_lim;              // kMagic + grid_occ_size
-    uint32_t sent_miss, sent_later, sent_none;   // sentinels in the biased index
+    uint32_t sent_miss;            // the sentinel in the biased index
     unsigned long long codes_b;
     // Grid layout (TSDFL_MAP_GRID): the codes of every brick of the bounding
     // box in brick order, so no rank is needed.  Brick up starts at
@@ -112,7 +117,7 @@ struct MapView {
     // grid_b = grid + 2 (sub_dim^3 - kMagic15) (bytes); grid_b is 0 without it.
     unsigned long long grid_b;
     uint32_t grid_uxy1;            // up_dim_2 - 1
-    uint32_t gsent_miss, gsent_later, gsent_none;   // sentinels in the grid's biased index
+    uint32_t gsent_miss;           // the sentinel in the grid's biased index
 };
 
 constexpr int kSentinels = 4;
@@ -184,6 +189,24 @@ static __device__ __forceinline__ void transform_point(const float* t, float x, 
 
 #endif  // __CUDACC__
 
+// Lookups a lane of the tiled kernels sums in one 64-bit word that holds the
+// values in its lower 57 bits (signed) and the hits above them.
+constexpr int kPackedLookups = 72;
+
+// Fixed-point scale 2^shift of the likelihood sums of n lookups of values up
+// to max_value in magnitude: at most 2^40, the sum of n + 1 below 2^62, and the
+// sum of kPackedLookups below 2^56 (without effect for a sigma of 0.042 m and
+// more; below, shorter scans get the scale a scan of 4,608 points has anyway).
+inline int fixed_shift(double max_value, double n)
+{
+    const double top = std::fmax(max_value, 1e-30);
+    const int sum = 62 - (int)std::ceil(std::log2(top * (n + 1.0)));
+    const int packed = 56 - (int)std::ceil(std::log2(top * kPackedLookups));
+    return std::min(40, std::min(sum, packed));
+}
+
+constexpr int kWorkWords = 8;
+
 // Kernel launchers (kernels.cu)
 struct EvalBuffers {
     const float* particles;  // P x 7
@@ -203,6 +226,7 @@ struct EvalBuffers {
     long long* lut_fx;       // kNumCodes fixed-point likelihoods
     float* lut_f;            // kNumCodes float likelihoods
     int32_t* counts;         // [0] = points in range
+    uint32_t* work;          // kWorkWords: item counters of the tiled kernels, 0 between launches
     double* partials;        // reduction partials
     double* sums;            // [0] weight sum, [1..9] pose sums
     float* weight_sum_f;     // [1]
