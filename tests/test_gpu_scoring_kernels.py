@@ -79,6 +79,13 @@ def same(ctx, dmap, parts, pts, tf=synth.IDENTITY_TF):
     assert ref["hits"].any() or parts.shape[0] * pts.shape[0] < 100   # a lookup or two may all miss
 
 
+SIZES = {False: ((2, 1), (15, 63), (16, 64), (17, 65), (33, 127), (64, 128), (65, 129), (250, 1024), (251, 1025),
+                 (20_000, 257), (40, 17_000)),
+         # at least kOrderFrom lookups: the spread kernel
+         True: ((400_009, 126), (400_000, 128), (395_001, 129), (800_000, 64), (800_001, 65), (16_401, 3203),
+                (16_384, 3072), (3001, 17_000))}
+
+
 @pytest.mark.parametrize("layout", list(LAYOUTS))
 @pytest.mark.parametrize("low", [(0.0, 0.0, 0.0), (-3.25, 1.5, -0.5)])
 @pytest.mark.parametrize("spread", [False, True])
@@ -88,8 +95,8 @@ def test_chunk_group_and_region_edges(ctx, layout, low, spread):
     coef, occ, codes = random_map(size, 0.1, low, 1)
     dmap = DeviceMap(ctx, coef, occ, codes=codes, **LAYOUTS[layout])
     assert dmap.info()["fast_index"]
-    for P, n in ((2, 1), (15, 63), (16, 64), (17, 65), (33, 127), (64, 128), (65, 129), (250, 1024), (251, 1025),
-                 (16_384, 200), (16_401, 257), (40, 17_000)):
+    for P, n in SIZES[spread]:
+        assert not spread or P * n >= 3 << 24
         same(ctx, dmap, cloud(spread, P, size, low, rng), scan(n, rng))
 
 
@@ -102,9 +109,9 @@ def test_bricks_that_alias_at_the_far_edge(ctx, layout):
     coef, occ, codes = random_map(size, 0.064, (0, 0, 0), 2)
     assert int(np.float32(21.0) / np.float32(0.064)) < coef.dim_x and coef.up_dim_x == 21
     dmap = DeviceMap(ctx, coef, occ, codes=codes, **LAYOUTS[layout])
-    for spread in (False, True):
-        parts = cloud(spread, 500, size, (0, 0, 0), rng)
-        parts[:250, :3] = np.array(size) - rng.random((250, 3)) * 0.2
+    for spread, P in ((False, 500), (True, 73_000)):
+        parts = cloud(spread, P, size, (0, 0, 0), rng)
+        parts[1:250, :3] = np.array(size) - rng.random((249, 3)) * 0.2
         same(ctx, dmap, parts, scan(700, rng))
 
 

@@ -76,7 +76,8 @@ struct tsdfl_ctx {
     size_t aux_bytes = 0;
     void* io = nullptr;          // device copies of host inputs (host API)
     size_t io_bytes = 0;
-    int32_t* status = nullptr;   // [0] sticky status, [1] per-evaluation status
+    int32_t* status = nullptr;   // [0] sticky status, [1] per-evaluation status, [2, 3] scratch
+    uint32_t* done = nullptr;    // the resampler's block counters (behind the status words)
     int32_t* h_status = nullptr; // pinned
     float* h_pose = nullptr;     // pinned, 8 floats
     uint32_t* h_count = nullptr; // pinned
@@ -635,10 +636,11 @@ int run_eval(tsdfl_ctx* c, const tsdfl_map* map, const tsdfl_model* mdl, float* 
     const int shift = fixed_shift(map->max_value, (double)N);
     const int npad = (int)align_up(N, 4);
     cudaStream_t s = c->stream;
+    const bool order = order_particles(P, N);
     rc = launch_pose_prepare(tf, d_particles, (int)P, d_points, (int)N, npad, max_range_sq, c_in, c_out, map->values,
-                             shift, b, s);
+                             shift, order, b, s);
     if (rc) return rc;
-    rc = launch_particle_order(d_particles, (int)P, b, s);
+    if (order) rc = launch_particle_order(d_particles, (int)P, b, s);
     if (rc) return rc;
     const bool tiled = !serial && map->view.storage == 0 && map->view.tiled && !(flags & TSDFL_EVAL_GENERIC);
     bool dense = map->occ != nullptr && !(tiled && map->grid);   // the grid layout needs no bitmap
@@ -689,10 +691,11 @@ int run_eval_sub(tsdfl_ctx* c, const tsdfl_map* map, const tsdfl_model* mdl, flo
     const int shift = fixed_shift(map->max_value, (double)K);
     const int npad = (int)align_up(N, 4);
     cudaStream_t s = c->stream;
+    const bool order = order_particles(P, K, kOrderFromSub);
     rc = launch_pose_prepare(tf, d_particles, (int)P, d_points, (int)N, npad, max_range_sq, c_in, c_out, map->values,
-                             shift, b, s);
+                             shift, order, b, s);
     if (rc) return rc;
-    rc = launch_particle_order(d_particles, (int)P, b, s);
+    if (order) rc = launch_particle_order(d_particles, (int)P, b, s);
     if (rc) return rc;
     if (c->timing) CUDA_TRY(cudaEventRecord(c->ev0, s));
     rc = launch_eval_subsample(map->view, mdl->a_hit, (int)P, (int)N, (int)K, seed, c_in, b, c->sm_count, s);
@@ -745,8 +748,9 @@ int tsdfl_ctx_create(int device, tsdfl_ctx** out)
     c->device = device;
     cudaError_t e = cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->own, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMalloc(&c->status, sizeof(int32_t) * 4);
-    if (e == cudaSuccess) e = cudaMemset(c->status, 0, sizeof(int32_t) * 4);
+    if (e == cudaSuccess) e = cudaMalloc(&c->status, sizeof(int32_t) * 8);
+    if (e == cudaSuccess) e = cudaMemset(c->status, 0, sizeof(int32_t) * 8);
+    c->done = reinterpret_cast<uint32_t*>(c->status + 4);
     if (e == cudaSuccess) e = cudaMallocHost(&c->h_status, sizeof(int32_t) * 4);
     if (e == cudaSuccess) e = cudaMallocHost(&c->h_pose, sizeof(float) * 8);
     if (e == cudaSuccess) e = cudaMallocHost(&c->h_count, sizeof(uint32_t) * 4);
@@ -1145,7 +1149,7 @@ int resample_systematic_host(tsdfl_ctx* c, const char* fn, const float* src, siz
     cudaStream_t s = c->stream;
     CUDA_TRY(cudaMemcpyAsync(d_src, src, sizeof(float) * stride * M, cudaMemcpyHostToDevice, s));
     rc = launch_resample_impl(nullptr, d_src + offset, (int)stride, M, u0, nullptr, d_idx, cap, d_cnt, c->rs_ws,
-                              c->status, s);
+                              c->done, c->status, s);
     if (rc) return rc;
     CUDA_TRY(cudaMemcpyAsync(c->h_count, d_cnt, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     if (cap) CUDA_TRY(cudaMemcpyAsync(idx_out, d_idx, sizeof(uint32_t) * cap, cudaMemcpyDeviceToHost, s));
@@ -1184,7 +1188,7 @@ int tsdfl_resample_systematic_device(tsdfl_ctx* c, const float* d_particles, siz
     rc = ensure_resample_ws(c, resample_workspace_bytes(M));
     if (rc) return rc;
     return launch_resample_impl(d_particles, d_particles + 6, 7, M, u0, d_particles_out, nullptr, cap, d_count,
-                                c->rs_ws, c->status, c->stream);
+                                c->rs_ws, c->done, c->status, c->stream);
 }
 
 int tsdfl_resample_residual_systematic(tsdfl_ctx* c, const float* weights, size_t M, float u0, uint32_t* idx_out,
@@ -1484,24 +1488,20 @@ void append_specs(tsdfl_batch* B, size_t i)
 
 cudaStream_t batch_stream(const tsdfl_batch* B) { return B->stream ? B->stream : B->ctx->stream; }
 
-// Scoring of every filter: the persistent launch, the filters that fill the
+// Scoring of every filter (pose_prepare_kernel has cleared their sums): the
+// persistent launch, the filters that fill the
 // GPU by themselves with the single-filter kernel (in their particle order for
 // a spread cloud), then the filters neither takes.
 int batch_score(tsdfl_batch* B, cudaStream_t s)
 {
     tsdfl_ctx* c = B->ctx;
-    for (size_t i = 0; i < B->f.size(); ++i) {
-        if (!B->per[i].tiled || B->per[i].big || B->f[i].N == 0) continue;
-        CUDA_TRY(cudaMemsetAsync(B->per[i].b.sum_fx, 0, sizeof(long long) * B->f[i].P, s));
-        CUDA_TRY(cudaMemsetAsync(B->per[i].b.hits, 0, sizeof(uint32_t) * B->f[i].P, s));
-    }
     int rc = launch_eval_batch(B->d_segs, B->kinds, B->d_counter, c->status, c->sm_count, s);
     if (rc) return rc;
-    for (size_t i = 0; i < B->f.size(); ++i) {   // pose_prepare_kernel cleared their sums
+    for (size_t i = 0; i < B->f.size(); ++i) {
         const tsdfl_filter& F = B->f[i];
         const tsdfl_batch::Per& q = B->per[i];
         if (!q.big || F.N == 0) continue;
-        rc = launch_particle_order(F.d_particles, (int)F.P, q.b, s);
+        if (order_particles(F.P, F.N)) rc = launch_particle_order(F.d_particles, (int)F.P, q.b, s);
         if (rc) return rc;
         for (size_t n0 = 0; n0 < F.N; n0 += q.pass) {
             size_t n1 = n0 + q.pass < F.N ? n0 + q.pass : F.N;
@@ -1524,6 +1524,17 @@ int batch_score(tsdfl_batch* B, cudaStream_t s)
     return TSDFL_OK;
 }
 
+// Clears every filter's sums for another batch_score of the same poses.
+int batch_clear(tsdfl_batch* B, cudaStream_t s)
+{
+    for (size_t i = 0; i < B->f.size(); ++i) {
+        if (!B->per[i].tiled || B->f[i].N == 0) continue;
+        CUDA_TRY(cudaMemsetAsync(B->per[i].b.sum_fx, 0, sizeof(long long) * B->f[i].P, s));
+        CUDA_TRY(cudaMemsetAsync(B->per[i].b.hits, 0, sizeof(uint32_t) * B->f[i].P, s));
+    }
+    return TSDFL_OK;
+}
+
 int batch_record(tsdfl_batch* B)
 {
     tsdfl_ctx* c = B->ctx;
@@ -1536,7 +1547,7 @@ int batch_record(tsdfl_batch* B)
         const float c_in = F.model.a_range * inv_max_range;
         int rc = launch_pose_prepare(F.tf, F.d_particles, (int)F.P, F.d_points, (int)F.N, q.npad,
                                      F.model.max_range * F.model.max_range, c_in, F.model.a_max, F.map->values,
-                                     q.shift, q.b, s);
+                                     q.shift, q.big && order_particles(F.P, F.N), q.b, s);
         if (rc) return rc;
     }
     int rc = batch_score(B, s);
@@ -1554,7 +1565,8 @@ int batch_record(tsdfl_batch* B)
         if (rc) return rc;
         if (F.d_u0 && F.d_resampled && F.P)
             rc = launch_resample_impl(F.d_particles, F.d_particles + 6, 7, F.P, 0.0f, F.d_resampled, nullptr,
-                                      F.resample_cap, F.d_count, q.rs_ws, sticky, s, F.d_u0);
+                                      F.resample_cap, F.d_count, q.rs_ws, q.b.work + kWorkResample, sticky, s,
+                                      F.d_u0);
         if (rc) return rc;
     }
     return TSDFL_OK;
@@ -1746,6 +1758,8 @@ int tsdfl_batch_autotune(tsdfl_batch* B, int* chunk_out, int* group_out, float* 
         if (rc) break;
         float t = 0;
         for (int rep = 0; rep < 3 && !rc; ++rep) {
+            rc = batch_clear(B, s);
+            if (rc) break;
             cudaEventRecord(e0, s);
             rc = batch_score(B, s);
             cudaEventRecord(e1, s);
@@ -2728,7 +2742,7 @@ int tsdfl_resample_systematic_static(tsdfl_ctx* c, const float* d_particles, siz
     rc = static_scratch(c->device, &scratch);
     if (rc) return rc;
     return launch_resample_impl(d_particles, d_particles + 6, 7, M, u0, d_particles_out, nullptr, cap, d_count,
-                                scratch, c->status, c->stream);
+                                scratch, c->done, c->status, c->stream);
 }
 
 }  // extern "C"

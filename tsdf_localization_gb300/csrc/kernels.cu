@@ -146,6 +146,8 @@ struct PointParams {
     float max_range_sq, c_in, c_out;
     const float* code_values;  // kNumCodes floats (device)
     int shift;                 // fixed-point scale 2^shift
+    int order;                 // a spread cloud's particles will be put in spatial order
+    int pose_warps;            // warps of a pose block that work
 };
 
 // Spatial order of the pair layout: the tiled kernels walk the scan in chunks
@@ -200,7 +202,8 @@ __device__ __forceinline__ void prepare_points_block(const PointParams& p, const
     __shared__ float4 s_ext[32];
     __shared__ int s_wide;
     if (threadIdx.x == 0) *b.status = 0;
-    for (int c = threadIdx.x; c < kCellBins; c += blockDim.x) b.phist[c] = 0;   // the particle order's histogram
+    if (p.order)
+        for (int c = threadIdx.x; c < kCellBins; c += blockDim.x) b.phist[c] = 0;   // the particle order's histogram
     {   // the cloud's x / y extent from a sample of the particles
         const float inf = __int_as_float(0x7f800000);
         float4 e = make_float4(inf, inf, -inf, -inf);
@@ -219,7 +222,7 @@ __device__ __forceinline__ void prepare_points_block(const PointParams& p, const
                 e = make_float4(fminf(e.x, v.x), fminf(e.y, v.y), fmaxf(e.z, v.z), fmaxf(e.w, v.w));
             }
             s_wide = fmaxf(e.z - e.x, e.w - e.y) > kWideCloud ? 1 : 0;   // no particles: -inf
-            b.counts[2] = s_wide;   // the particles are put in spatial order too
+            b.counts[2] = p.order ? s_wide : 0;   // the particles are put in spatial order too
             for (int k = 0; k < kWorkWords; ++k) b.work[k] = 0u;
             b.cloud_ext[0] = e;
         }
@@ -406,13 +409,15 @@ struct Tf16 {
 // and lane 3p + r forms row r of the 3 x 4 laser pose, so the FP64 latency of
 // the three sincos is spread over three lanes.  Also zeros in the scoring
 // sums, so no memset breaks the chain of kernels.  `blk` numbers the pose
-// blocks of pose_prepare_kernel.
-__device__ __forceinline__ void pose_block(int blk, const float* particles, int P, const Tf16& tf, float* pose12,
-                                           float* trig6, long long* sum_fx, uint32_t* hits)
+// blocks of pose_prepare_kernel; of each, `warps` warps work (a small cloud is
+// spread over the SMs, whose FP64 pipes are what it waits for).
+__device__ __forceinline__ void pose_block(int blk, int warps, const float* particles, int P, const Tf16& tf,
+                                           float* pose12, float* trig6, long long* sum_fx, uint32_t* hits)
 {
+    if ((int)(threadIdx.x >> 5) >= warps) return;
     const int lane = threadIdx.x & 31;
     const int slot = lane / 3, k = lane - 3 * slot;
-    const int i = (blk * (kPoseThreads / 32) + (int)(threadIdx.x >> 5)) * kPoseSlots + slot;
+    const int i = (blk * warps + (int)(threadIdx.x >> 5)) * kPoseSlots + slot;
     const bool active = slot < kPoseSlots && i < P;
     if (active && k == 0) {   // the tiled kernel's per-particle sums start at zero
         sum_fx[i] = 0;
@@ -464,7 +469,7 @@ __global__ void __launch_bounds__(kPoseThreads) pose_prepare_kernel(Tf16 tf, Poi
 {
     chain_enter();
     if (blockIdx.x == 0) prepare_points_block(p, b);
-    else pose_block((int)blockIdx.x - 1, p.particles, p.P, tf, b.pose12, b.trig6, b.sum_fx, b.hits);
+    else pose_block((int)blockIdx.x - 1, p.pose_warps, p.particles, p.P, tf, b.pose12, b.trig6, b.sum_fx, b.hits);
 }
 
 struct EvalParams {
@@ -1678,16 +1683,14 @@ __global__ void norm_partial_kernel(NormParams q, EvalBuffers b, const double* s
 }
 
 // Final weight sum, the "No particle is valid!" check (tsdf_evaluator.cpp:159)
-// and the mean pose with circular means of the angles (:219-221).  One block
-// of kNormBlocks threads: thread t takes block t's partial sums (nb blocks ran),
+// and the mean pose with circular means of the angles (:219-221), by one block
+// of kNormThreads threads: thread t takes block t's partial sums (nb blocks ran),
 // then a fixed reduction tree (so the result does not depend on timing); the
 // position and the three angles are formed by four threads side by side.
-__global__ void __launch_bounds__(kNormBlocks) norm_final_kernel(EvalBuffers b, float* pose_out, int nb)
+__device__ __forceinline__ void norm_final_block(const EvalBuffers& b, float* pose_out, int nb,
+                                                 double (*red)[kNormThreads], double (*red2)[kNormSumsParts])
 {
-    chain_enter();
     static_assert(kNormBlocks == kNormThreads, "one partial per thread");
-    __shared__ double red[kNormSums][kNormThreads];
-    __shared__ double red2[kNormSums][kNormSumsParts];
     __shared__ double s[kNormSums];
     const int t = threadIdx.x;
     double acc[kNormSums];
@@ -1715,26 +1718,54 @@ __global__ void __launch_bounds__(kNormBlocks) norm_final_kernel(EvalBuffers b, 
     }
 }
 
-// particles[i].second = raw / weight_sum (tsdf_evaluator.cpp:203), skipped when
-// the sum was degenerate so the caller's particles stay untouched.
-// Also the last step of an evaluation: thread 0 carries its device status into
+// Also the last step of an evaluation: one thread carries its device status into
 // the sticky status word (when one is given and still clear).
 __device__ __forceinline__ void fold_status(const int32_t* ev, int32_t* sticky)
 {
-    if (sticky && blockIdx.x == 0 && threadIdx.x == 0) {
-        const int v = *ev;
-        if (v && *sticky == 0) *sticky = v;
-    }
+    const int v = *ev;
+    if (sticky && v && *sticky == 0) *sticky = v;
 }
 
-__global__ void normalize_kernel(int P, EvalBuffers b, float* particles_out, int32_t* sticky)
+// particles[i].second = raw / weight_sum (tsdf_evaluator.cpp:203), skipped when
+// the sum was degenerate so the caller's particles stay untouched.  Block 0
+// forms the final sums and the mean pose meanwhile; the others add the weight
+// sum's partials themselves, in its order, instead of waiting for a launch
+// between.
+__global__ void __launch_bounds__(kNormThreads) normalize_kernel(int P, EvalBuffers b, float* particles_out,
+                                                                 float* pose_out, int nb, int32_t* sticky)
 {
     chain_enter();
-    fold_status(b.status, sticky);
-    if (*b.status == TSDFL_ERR_DEGENERATE) return;
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P) return;
-    particles_out[7 * (size_t)i + 6] = __fdiv_rn(b.raw[i], b.weight_sum_f[0]);
+    __shared__ double red[kNormSums][kNormThreads];
+    __shared__ double red2[kNormSums][kNormSumsParts];
+    const int t = threadIdx.x;
+    if (blockIdx.x == 0) {
+        norm_final_block(b, pose_out, nb, red, red2);
+        if (t == 0) fold_status(b.status, sticky);
+        return;
+    }
+    red[0][t] = t < nb ? b.partials[t * kNormSums] : 0.0;
+    __syncthreads();
+    if (t < kNormSumsParts) {   // block_sums10's order
+        double v = 0.0;
+        for (int j = 0; j < kNormThreads / kNormSumsParts; ++j) v += red[0][t + kNormSumsParts * j];
+        red2[0][t] = v;
+    }
+    __syncthreads();
+    double sum = 0.0;
+    for (int j = 0; j < kNormSumsParts; ++j) sum += red2[0][j];
+    const float w = (float)sum;
+    if (!(w != 0.0f) || !isfinite(sum)) return;
+    const int step = (int)(gridDim.x - 1) * kNormThreads;
+    for (int i = (int)(blockIdx.x - 1) * kNormThreads + t; i < P; i += step)
+        particles_out[7 * (size_t)i + 6] = __fdiv_rn(b.raw[i], w);
+}
+
+__global__ void __launch_bounds__(kNormThreads) norm_final_kernel(EvalBuffers b, float* pose_out, int nb)
+{
+    chain_enter();
+    __shared__ double red[kNormSums][kNormThreads];
+    __shared__ double red2[kNormSums][kNormSumsParts];
+    norm_final_block(b, pose_out, nb, red, red2);
 }
 
 // Log-domain normalisation (TSDFL_NORM_LOG), after norm_partial/final have
@@ -1787,7 +1818,7 @@ __global__ void __launch_bounds__(kNormBlocks) log_final_kernel(EvalBuffers b)
 
 __global__ void normalize_log_kernel(int P, EvalBuffers b, float* particles_out, int32_t* sticky)
 {
-    fold_status(b.status, sticky);
+    if (blockIdx.x == 0 && threadIdx.x == 0) fold_status(b.status, sticky);
     if (*b.status == TSDFL_ERR_DEGENERATE) return;
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P) return;
@@ -1815,7 +1846,8 @@ struct SumsChunk {
     int b;                   // binade of every serial sum the chunk touches, or kNoBinade
     int delta;               // increment for an odd start minus R0 (+-1 at the first tie, else 0)
     int ok;                  // no weight reaches 2^(b+1): R0 and delta hold
-    int par;                 // the chunk's sums are written by resample_chunk_write_kernel
+    int par;                 // the chunk's sums follow from P and its increments
+    double start;            // the sum before the chunk (par clear)
 };
 
 struct Segment {
@@ -1833,10 +1865,14 @@ struct ResampleWs {
     int* nseg;
     int* exact_ok;          // 1 when the parallel path reproduces the serial one
     long long* total;
+    double* reach;          // the segments describe the draws below this
     int* serial;            // 1 when only the literal loop reproduces it
     double* sums;           // M serial double prefix sums (aliases cdf; used when !exact_ok)
     const float* u0p;       // the draw in device memory (replaces u0 when set)
     double* tile_dsum;      // tiles: double sum of each scan tile's weights (any order)
+    int* tile_flag;         // tiles: kTileInexact, kTileWild
+    int* err;               // the literal loop would never finish
+    uint32_t* done;         // two block counters, 0 between launches
     SumsChunk* chunks;      // ceil(M / kSumsChunk)
 };
 
@@ -1861,13 +1897,40 @@ __device__ __forceinline__ long long weight_fx52(float w)
     return mant >> -sh;
 }
 
+// Whether the calling block is the grid's last to get here (the same on every
+// thread): its writes before the call are visible to the last block, which may
+// read the others' with __ldcg.  The counter returns to 0.
+__device__ __forceinline__ bool last_block(uint32_t* counter)
+{
+    __shared__ int s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicInc(counter, gridDim.x - 1u) == gridDim.x - 1u;
+    __syncthreads();
+    if (s_last) __threadfence();
+    return s_last != 0;
+}
+
+constexpr int kTileInexact = 1;   // a weight is not a multiple of 2^-52 (or too large)
+constexpr int kTileWild = 2;      // a weight is negative or not finite
+
+__device__ void offsets_warp(int tiles, const ResampleWs& ws);
+__device__ double build_segments(int M, float u0, double s_total, const ResampleWs& ws);
+
 // Tile-local inclusive scan of the fixed-point weights (exact integers).
-// Also the tile's double sum of the weights for the fallback below, and
-// *ws.serial for a negative or non-finite weight (only the literal loop
-// reproduces those).
-__global__ void resample_scan_kernel(const float* w, int stride, int M, ResampleWs ws)
+// Also the tile's double sum of the weights for the fallback below, and its
+// flags.  Block `tiles` describes the draws below 2 as segments meanwhile (the
+// fixed-point sums stay below that); the last block to finish then forms the
+// tiles' offsets.
+__global__ void __launch_bounds__(kScanThreads) resample_scan_kernel(const float* w, int stride, int M, float u0,
+                                                                     ResampleWs ws)
 {
     chain_enter();
+    if (blockIdx.x == gridDim.x - 1) {
+        if (threadIdx.x == 0) *ws.reach = build_segments(M, ws.u0p ? *ws.u0p : u0, 2.0, ws);
+        if (last_block(ws.done) && threadIdx.x < 32) offsets_warp((int)gridDim.x - 1, ws);
+        return;
+    }
     __shared__ long long warp_tot[kScanThreads / 32];
     __shared__ double warp_d[kScanThreads / 32];
     __shared__ int bad, wild;
@@ -1917,8 +1980,8 @@ __global__ void resample_scan_kernel(const float* w, int stride, int M, Resample
         ws.tile_dsum[blockIdx.x] = d;
     }
     __syncthreads();
-    if (threadIdx.x == 0 && bad) atomicExch(ws.exact_ok, 0);
-    if (threadIdx.x == 0 && wild) atomicExch(ws.serial, 1);
+    if (threadIdx.x == 0) ws.tile_flag[blockIdx.x] = (bad ? kTileInexact : 0) | (wild ? kTileWild : 0);
+    if (last_block(ws.done) && threadIdx.x < 32) offsets_warp((int)gridDim.x - 1, ws);
 }
 
 // 2^k for -1022 <= k <= 1023, exactly.
@@ -1936,12 +1999,12 @@ __device__ __forceinline__ double binade_value(unsigned long long V, int b)
 // Builds the piecewise-arithmetic description of the reference's float draw
 // sequence U_{k+1} = (float)((double)U_k + 1.0/M) (novel_resampling.h:59-63)
 // for all draws below s_total: inside one binade of float the step is constant
-// except near its top, where single steps are taken literally.  False when it
-// cannot (a step that would depend on the parity of U, a draw that stops
+// except near its top, where single steps are taken literally.  Returns how far
+// the description reaches: s_total (or the first draw past it), or less when it
+// ends before (a step that would depend on the parity of U, a draw that stops
 // advancing, more than kMaxSegments pieces).  Scalings by powers of two only.
-__device__ bool build_segments(int M, float u0, double s_total, ResampleWs ws)
+__device__ double build_segments(int M, float u0, double s_total, const ResampleWs& ws)
 {
-    bool ok = true;
     const double inv_m = 1.0 / (double)M;
     // 1/M = Mi 2^(Ei - 52): the binade arithmetic below is integer work on the
     // doubles' bits (one lane walks the binades; GB300's FP64 pipe is narrow)
@@ -1954,14 +2017,14 @@ __device__ bool build_segments(int M, float u0, double s_total, ResampleWs ws)
     int ns = 0;
     if (!(s_total >= 0.0) || !(s_total < INFINITY)) {   // no sum of non-negative finite weights
         *ws.nseg = 0;
-        return false;
+        return 0.0;
     }
     // the draws' and the sums' doubles are compared on their bits (a sum here
     // is >= +0, and a double >= +0 orders like its bits as a signed integer)
     const long long s_bits = __double_as_longlong(s_total);
     const long long kFltMinBits = 0x3810000000000000ll;   // 2^-126, the smallest normal float
     for (int iter = 0; __double_as_longlong(U) < s_bits; ++iter) {
-        if (ns == kMaxSegments || iter > 4 * kMaxSegments) { ok = false; break; }
+        if (ns == kMaxSegments || iter > 4 * kMaxSegments) break;
         bool regular = false;
         long long cnt = 0;
         int e = 0;
@@ -1991,11 +2054,11 @@ __device__ bool build_segments(int M, float u0, double s_total, ResampleWs ws)
                 }
                 low = Y & kMask29;
             }
-            if (low == kHalf29) { ok = false; break; }   // step would depend on the parity of U
+            if (low == kHalf29) break;   // step would depend on the parity of U
             if (!big) {
                 // delta = rint(Y g / u) u = R 2^29 g
                 const unsigned long long R = (Y >> 29) + (low > kHalf29 ? 1ull : 0ull);
-                if (R == 0) { ok = false; break; }        // U would stop advancing
+                if (R == 0) break;        // U would stop advancing
                 D = R << 29;
                 {   // delta = R 2^(e-23), built from its bits (R < 2^25)
                     const int lz = __clzll((long long)R);
@@ -2028,28 +2091,26 @@ __device__ bool build_segments(int M, float u0, double s_total, ResampleWs ws)
             ++ns;
             j += 1;
             double next = (double)(float)(U + inv_m);
-            if (!(next > U)) { ok = false; break; }   // U stopped advancing
+            if (!(next > U)) break;   // U stopped advancing
             U = next;
         }
     }
     *ws.nseg = ns;
-    return ok;
+    return U;
 }
 
-// Builds the piecewise-arithmetic description of the reference's float draw
-// sequence U_{k+1} = (float)((double)U_k + 1.0/M) (novel_resampling.h:59-63):
-// inside one binade of float the step is constant except near its top, where
-// single steps are taken literally.  One warp: the lanes form the tiles'
-// prefix offsets, lane 0 walks the binades (scalings by powers of two only).
-__global__ void resample_segments_kernel(int M, float u0, int tiles, ResampleWs ws)
+// The tiles' prefix offsets, and which of the forms below reproduces the
+// reference (exact_ok, serial).
+__device__ void offsets_warp(int tiles, const ResampleWs& ws)
 {
-    chain_enter();
-    if (ws.u0p) u0 = *ws.u0p;
     const int lane = threadIdx.x & 31;
-    if (threadIdx.x >= 32 || blockIdx.x != 0) return;
     const int per = (tiles + 31) / 32, t0 = min(tiles, lane * per), t1 = min(tiles, t0 + per);
     long long loc = 0;
-    for (int t = t0; t < t1; ++t) loc += ws.tile_sums[t];
+    int flags = 0;
+    for (int t = t0; t < t1; ++t) {
+        loc += __ldcg(ws.tile_sums + t);
+        flags |= __ldcg(ws.tile_flag + t);
+    }
     long long x = loc;   // inclusive scan over the lanes (exact integers)
     for (int o = 1; o < 32; o <<= 1) {
         const long long y = __shfl_up_sync(0xffffffffu, x, o);
@@ -2058,14 +2119,16 @@ __global__ void resample_segments_kernel(int M, float u0, int tiles, ResampleWs 
     long long off = x - loc;
     for (int t = t0; t < t1; ++t) {
         ws.tile_off[t] = off;
-        off += ws.tile_sums[t];
+        off += __ldcg(ws.tile_sums + t);
     }
     const long long acc = __shfl_sync(0xffffffffu, x, 31);
+    flags = __reduce_or_sync(0xffffffffu, (unsigned)flags);
     if (lane != 0) return;
     *ws.total = acc;
-    if (acc >= (1ll << 53)) *ws.exact_ok = 0;   // partial sums >= 2 may round in the serial double sum
-    if (!*ws.exact_ok) { *ws.nseg = 0; return; }
-    if (!build_segments(M, u0, ldexp((double)acc, -52), ws)) *ws.exact_ok = 0;
+    *ws.err = 0;
+    *ws.serial = flags & kTileWild ? 1 : 0;
+    // partial sums >= 2 may round in the serial double sum
+    *ws.exact_ok = !(flags & kTileInexact) && acc < (1ll << 53) && __ldcg(ws.reach) >= ldexp((double)acc, -52);
 }
 
 // Number of draws U_j below s (the count the serial loop has emitted once its
@@ -2131,19 +2194,32 @@ __device__ __forceinline__ long long count_below_fx(const Segment* seg, int ns, 
     return g.j0 + (long long)((S - A + R - 1ull) / R);
 }
 
+// Copies particle m (7 floats) to the output rows [lo, hi) below cap, or writes
+// its index there.
+__device__ __forceinline__ void copy_rows(const float* particles, int m, long long lo, long long hi, long long cap,
+                                          float* out, uint32_t* idx_out)
+{
+    for (long long j = lo; j < hi && j < cap; ++j) {
+        if (idx_out) idx_out[j] = (uint32_t)m;
+        if (out) {
+            const float* src = particles + 7 * (size_t)m;
+            float* dst = out + 7 * (size_t)j;
+            for (int k = 0; k < 7; ++k) dst[k] = src[k];
+        }
+    }
+}
+
 // Particle m receives the draws in [cdf_{m-1}, cdf_m) (novel_resampling.h:52-68):
 // writes their indices and, when asked, copies of the particle.
-__global__ void resample_assign_kernel(const float* particles, int M, float* out, uint32_t* idx_out, long long cap,
-                                       uint32_t* count_out, ResampleWs ws, int32_t* status)
+__device__ __forceinline__ void assign_block(const float* particles, int M, float* out, uint32_t* idx_out,
+                                             long long cap, uint32_t* count_out, const ResampleWs& ws, int32_t* status,
+                                             Segment* seg, int per)
 {
-    chain_enter();
-    __shared__ Segment seg[kMaxSegments];
-    if (!*ws.exact_ok) return;
     const int ns = *ws.nseg;
     for (int k = threadIdx.x; k < ns; k += blockDim.x) seg[k] = ws.segs[k];
     __syncthreads();
-    int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= M) return;
+    const int m = (int)blockIdx.x * per + (int)threadIdx.x;
+    if ((int)threadIdx.x >= per || m >= M) return;
     const long long c_hi_fx = ws.cdf[m] + ws.tile_off[m / kScanTile];
     long long c_lo_fx = 0;
     if (m > 0) c_lo_fx = ws.cdf[m - 1] + ws.tile_off[(m - 1) / kScanTile];
@@ -2153,14 +2229,7 @@ __global__ void resample_assign_kernel(const float* particles, int M, float* out
         *count_out = (uint32_t)hi;
         if (hi > cap) atomicExch(status, TSDFL_ERR_CAPACITY);
     }
-    for (long long j = lo; j < hi && j < cap; ++j) {
-        if (idx_out) idx_out[j] = (uint32_t)m;
-        if (out) {
-            const float* src = particles + 7 * (size_t)m;
-            float* dst = out + 7 * (size_t)j;
-            for (int k = 0; k < 7; ++k) dst[k] = src[k];
-        }
-    }
+    copy_rows(particles, m, lo, hi, cap, out, idx_out);
 }
 
 constexpr int kChainTile = 2048;
@@ -2183,14 +2252,15 @@ constexpr int kChainTile = 2048;
 // per binade the running sum crosses).  Such a chunk's increment depends on
 // the sum before it only through that sum's parity, at the chunk's first tie,
 // so it is formed for both parities by one block per chunk
-// (resample_chunk_transfer_kernel); one block then chains the chunks' starts,
-// walking the others weight by weight (resample_sums_kernel), after which one
-// block per chunk writes the chained chunks' sums (resample_chunk_write_kernel).
+// (chunk_transfer_block); the last block to finish then chains the chunks'
+// starts, walking the others weight by weight (serial_sums_block), after which one
+// block per chunk forms the chained chunks' sums and gives every particle its
+// draws (resample_finish_kernel).
 // The chain verifies each transfer it applies (the start in the chunk's binade,
 // the end below the binade's top), so the margin only decides speed, never the
 // result.  Negative or non-finite weights set *ws.serial: only the literal loop
 // reproduces them.  With s monotone, the draws each particle emits then follow
-// from the draw segments in parallel (resample_fallback_assign_kernel).
+// from the draw segments in parallel.
 // One weight in units u = 2^(b-52) of the running sum's binade [2^b, 2^(b+1)),
 // from the float's bits alone (integer shifts, no FP64 operation): q =
 // floor(w / u), whether the remainder is exactly half a unit (a tie) or above
@@ -2355,6 +2425,11 @@ __device__ __forceinline__ double block_sum_d(double v, double* red)
     return t;
 }
 
+struct SumsShared {   // binade_increments' reductions
+    unsigned long long sum[kSumsThreads / 32];
+    ParityPrefix par[kSumsThreads / 32];
+};
+
 // Stages chunk c's weights in shared memory; returns its length.
 __device__ __forceinline__ int stage_chunk(const float* __restrict__ w, int stride, int M, int c, float* sw)
 {
@@ -2367,16 +2442,11 @@ __device__ __forceinline__ int stage_chunk(const float* __restrict__ w, int stri
 // tiles' double sums, widened by far more than their rounding), and for a
 // chunk inside one binade its increment R0 from an even start and the change
 // delta for an odd one.
-__global__ void __launch_bounds__(kSumsThreads) resample_chunk_transfer_kernel(const float* __restrict__ w,
-                                                                               int stride, int M, ResampleWs ws)
+__device__ __forceinline__ void chunk_transfer_block(const float* __restrict__ w, int stride, int M,
+                                                     const ResampleWs& ws, float* sw, SumsShared& sh)
 {
-    chain_enter();
-    __shared__ float sw[kSumsChunk];
-    __shared__ unsigned long long red_sum[kSumsThreads / 32];
-    __shared__ ParityPrefix red_par[kSumsThreads / 32];
     __shared__ double red_d[kSumsThreads / 32];
     __shared__ int s_b, s_first, s_big;
-    if (*ws.exact_ok || *ws.serial) return;
     const int c = blockIdx.x, tid = threadIdx.x;
     constexpr int kTilesPerChunk = kSumsChunk / kScanTile;
     const int tiles = (M + kScanTile - 1) / kScanTile;
@@ -2402,6 +2472,7 @@ __global__ void __launch_bounds__(kSumsThreads) resample_chunk_transfer_kernel(c
         k.delta = 0;
         k.R0 = 0;
         k.P = 0;
+        k.start = 0.0;
     }
     __syncthreads();
     const int b = s_b;
@@ -2409,7 +2480,7 @@ __global__ void __launch_bounds__(kSumsThreads) resample_chunk_transfer_kernel(c
     const int t = stage_chunk(w, stride, M, c, sw);
     __syncthreads();
     BinadeRun x;
-    binade_increments(sw, 0, t, b, 0u, x, red_par, red_sum);
+    binade_increments(sw, 0, t, b, 0u, x, sh.par, sh.sum);
     bool big = false;
     for (int j = 0; j < kSumsItems; ++j) {
         big |= x.big[j];
@@ -2428,7 +2499,7 @@ __global__ void __launch_bounds__(kSumsThreads) resample_chunk_transfer_kernel(c
 
 __device__ void systematic_chain_block(const float* __restrict__ w, int stride, int M, float u0,
                                        uint32_t* __restrict__ cnt, uint32_t* __restrict__ off,
-                                       unsigned long long* total, int* err);
+                                       unsigned long long* total, int* err, unsigned char* buf);
 
 // The chain: one block walks the chunks in order, applying the transfers of
 // chunks inside one binade (thread 0, checked) and forming the others' sums
@@ -2436,11 +2507,9 @@ __device__ void systematic_chain_block(const float* __restrict__ w, int stride, 
 // segments.  Where only the literal loop reproduces the reference (*ws.serial:
 // set by the scan for negative or non-finite weights, or here when the draws
 // cannot be described), the block walks that instead.
-__device__ void serial_sums_block(const float* __restrict__ w, int stride, int M, float u0, ResampleWs ws)
+__device__ void serial_sums_block(const float* __restrict__ w, int stride, int M, float u0, const ResampleWs& ws,
+                                  float* sw, SumsShared& sh)
 {
-    __shared__ float sw[kSumsChunk];
-    __shared__ unsigned long long red_sum[kSumsThreads / 32];
-    __shared__ ParityPrefix red_par[kSumsThreads / 32];
     __shared__ double s_s, s_prev;
     __shared__ int s_pos, s_e, s_c;
     const int tid = threadIdx.x;
@@ -2456,17 +2525,20 @@ __device__ void serial_sums_block(const float* __restrict__ w, int stride, int M
             int c = s_c;
             double sum = s_s;
             for (; c < chunks; ++c) {
-                SumsChunk& k = ws.chunks[c];
-                if (k.b == kNoBinade || !k.ok || !(sum > 0.0) || binade_of(sum) != k.b) break;
+                SumsChunk& k = ws.chunks[c];   // another block's transfer: read past the L1
+                const int kb = __ldcg(&k.b);
+                if (kb == kNoBinade || !__ldcg(&k.ok) || !(sum > 0.0) || binade_of(sum) != kb) break;
                 const unsigned long long P = binade_units(sum);
-                const unsigned long long E = P + k.R0 + ((P & 1ull) ? (unsigned long long)(long long)k.delta : 0ull);
+                const unsigned long long E =
+                    P + __ldcg(&k.R0) + ((P & 1ull) ? (unsigned long long)(long long)__ldcg(&k.delta) : 0ull);
                 if (E >= LIM) break;
                 k.P = P;
                 k.par = 1;
-                sum = binade_value(E, k.b);
+                sum = binade_value(E, kb);
             }
             s_c = c;
             s_s = sum;
+            if (c < chunks) ws.chunks[c].start = sum;
         }
         __syncthreads();
         const int c = s_c;
@@ -2500,7 +2572,7 @@ __device__ void serial_sums_block(const float* __restrict__ w, int stride, int M
             const int b = binade_of(s);   // s in [2^b, 2^(b+1))
             const unsigned long long P0 = binade_units(s);
             BinadeRun x;
-            binade_increments(sw, pos, t, b, (uint32_t)(P0 & 1ull), x, red_par, red_sum);
+            binade_increments(sw, pos, t, b, (uint32_t)(P0 & 1ull), x, sh.par, sh.sum);
             for (int j = 0; j < kSumsItems; ++j) {
                 const int i = pos + kSumsItems * tid + j;
                 const unsigned long long before = x.incl[j] - x.r[j];
@@ -2531,91 +2603,91 @@ __device__ void serial_sums_block(const float* __restrict__ w, int stride, int M
         if (tid == 0) s_c = c + 1;
         __syncthreads();
     }
-    if (tid == 0 && !build_segments(M, u0, s_s, ws)) *ws.serial = 1;   // s_s: the total
+    if (tid == 0 && !(build_segments(M, u0, s_s, ws) >= s_s)) *ws.serial = 1;   // s_s: the total
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(kSumsThreads) resample_sums_kernel(const float* __restrict__ w, int stride, int M,
-                                                                     float u0, ResampleWs ws, uint32_t* cnt,
-                                                                     uint32_t* off, unsigned long long* total,
-                                                                     int* err)
-{
-    chain_enter();
-    if (*ws.exact_ok) return;
-    if (ws.u0p) u0 = *ws.u0p;
-    if (!*ws.serial) serial_sums_block(w, stride, M, u0, ws);
-    if (*ws.serial) systematic_chain_block(w, stride, M, u0, cnt, off, total, err);
-}
+// The draws' copies on the exact path (`per` particles a block); else the first part of the fallbacks: the
+// chunks' transfers, then (the last block) their chain, or the literal loop.
+constexpr int kAssignBytes = kMaxSegments * (int)sizeof(Segment);
+static_assert(kAssignBytes >= kSumsChunk * (int)sizeof(float) && kAssignBytes >= 3 * 2048 * 4, "one buffer for all");
 
-// One block per chained chunk: its sums from the start the chain gave it.
-__global__ void __launch_bounds__(kSumsThreads) resample_chunk_write_kernel(const float* __restrict__ w, int stride,
-                                                                            int M, ResampleWs ws)
+__global__ void __launch_bounds__(kSumsThreads) resample_assign_kernel(const float* particles,
+                                                                       const float* __restrict__ w, int stride, int M,
+                                                                       float u0, float* out, uint32_t* idx_out,
+                                                                       long long cap, uint32_t* count_out,
+                                                                       ResampleWs ws, uint32_t* cnt, uint32_t* off,
+                                                                       int32_t* status, int per)
 {
     chain_enter();
-    __shared__ float sw[kSumsChunk];
-    __shared__ unsigned long long red_sum[kSumsThreads / 32];
-    __shared__ ParityPrefix red_par[kSumsThreads / 32];
-    if (*ws.exact_ok || *ws.serial) return;
-    const int c = blockIdx.x;
-    const SumsChunk k = ws.chunks[c];
-    if (!k.par) return;
-    const int t = stage_chunk(w, stride, M, c, sw);
-    __syncthreads();
-    BinadeRun x;
-    binade_increments(sw, 0, t, k.b, (uint32_t)(k.P & 1ull), x, red_par, red_sum);
-    const int c0 = c * kSumsChunk;
-    for (int j = 0; j < kSumsItems; ++j) {
-        const int i = kSumsItems * threadIdx.x + j;
-        if (x.valid[j]) ws.sums[c0 + i] = binade_value(k.P + x.incl[j], k.b);
+    __shared__ __align__(16) unsigned char buf[kAssignBytes];
+    __shared__ SumsShared sh;
+    if (*ws.exact_ok) {
+        assign_block(particles, M, out, idx_out, cap, count_out, ws, status, reinterpret_cast<Segment*>(buf), per);
+        return;
     }
+    float* sw = reinterpret_cast<float*>(buf);
+    if (!*ws.serial && (int)blockIdx.x < (M + kSumsChunk - 1) / kSumsChunk) chunk_transfer_block(w, stride, M, ws, sw, sh);
+    if (!last_block(ws.done + 1)) return;
+    if (ws.u0p) u0 = *ws.u0p;
+    if (!*ws.serial) serial_sums_block(w, stride, M, u0, ws, sw, sh);
+    if (*ws.serial)
+        systematic_chain_block(w, stride, M, u0, cnt, off, reinterpret_cast<unsigned long long*>(ws.total), ws.err, buf);
 }
 
 __device__ void scatter_block(const float* particles, int M, const uint32_t* cnt, const uint32_t* off,
                               const unsigned long long* total, const int* err, float* out, uint32_t* idx_out,
                               long long cap, uint32_t* count_out, int32_t* status);
 
-// The fallbacks' assignment: from the literal loop's counts and offsets
-// (*ws.serial), else particle m receives the draws in [s_{m-1}, s_m) of the
-// serial double sums.
-__global__ void resample_fallback_assign_kernel(const float* particles, int M, float* out, uint32_t* idx_out,
-                                                long long cap, uint32_t* count_out, ResampleWs ws, int32_t* status,
-                                                const uint32_t* cnt, const uint32_t* off,
-                                                const unsigned long long* total, const int* err)
+// The fallbacks' second part (at once over on the exact path): from the literal
+// loop's counts and offsets (*ws.serial), else one block per chunk -- the chunk's
+// serial double sums from the start the chain gave it, or as the chain stored
+// them, and particle m receives the draws in [s_{m-1}, s_m).
+__global__ void __launch_bounds__(kSumsThreads) resample_finish_kernel(const float* particles,
+                                                                       const float* __restrict__ w, int stride, int M,
+                                                                       float* out, uint32_t* idx_out, long long cap,
+                                                                       uint32_t* count_out, ResampleWs ws,
+                                                                       const uint32_t* cnt, const uint32_t* off,
+                                                                       int32_t* status)
 {
     chain_enter();
-    __shared__ Segment seg[kMaxSegments];
+    __shared__ float sw[kSumsChunk];
+    __shared__ SumsShared sh;
     if (*ws.exact_ok) return;
     if (*ws.serial) {
-        scatter_block(particles, M, cnt, off, total, err, out, idx_out, cap, count_out, status);
+        scatter_block(particles, M, cnt, off, reinterpret_cast<const unsigned long long*>(ws.total), ws.err, out, idx_out,
+                      cap, count_out, status);
         return;
     }
-    const int ns = *ws.nseg;
-    for (int k = threadIdx.x; k < ns; k += blockDim.x) seg[k] = ws.segs[k];
-    __syncthreads();
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= M) return;
-    const long long lo = m > 0 ? count_below(seg, ns, ws.sums[m - 1]) : 0;
-    const long long hi = count_below(seg, ns, ws.sums[m]);
-    if (m == M - 1) {
-        *count_out = (uint32_t)hi;
-        if (hi > cap) atomicExch(status, TSDFL_ERR_CAPACITY);
+    const int c = blockIdx.x;
+    if (c >= (M + kSumsChunk - 1) / kSumsChunk) return;
+    const SumsChunk k = ws.chunks[c];
+    const int c0 = c * kSumsChunk, t = min(kSumsChunk, M - c0), ns = *ws.nseg;
+    double s[kSumsItems + 1];   // the sums before and after this thread's items
+    if (k.par) {
+        stage_chunk(w, stride, M, c, sw);
+        __syncthreads();
+        BinadeRun x;
+        binade_increments(sw, 0, t, k.b, (uint32_t)(k.P & 1ull), x, sh.par, sh.sum);
+        s[0] = binade_value(k.P + x.incl[0] - x.r[0], k.b);
+        for (int j = 0; j < kSumsItems; ++j) s[j + 1] = binade_value(k.P + x.incl[j], k.b);
+    } else {
+        const int i = kSumsItems * (int)threadIdx.x;
+        s[0] = i == 0 ? k.start : (i <= t ? ws.sums[c0 + i - 1] : 0.0);
+        for (int j = 0; j < kSumsItems; ++j) s[j + 1] = i + j < t ? ws.sums[c0 + i + j] : 0.0;
     }
-    for (long long j = lo; j < hi && j < cap; ++j) {
-        if (idx_out) idx_out[j] = (uint32_t)m;
-        if (out) {
-            const float* src = particles + 7 * (size_t)m;
-            float* dst = out + 7 * (size_t)j;
-            for (int k = 0; k < 7; ++k) dst[k] = src[k];
+    const int i = kSumsItems * (int)threadIdx.x;
+    long long lo = i < t ? count_below(ws.segs, ns, s[0]) : 0;
+    for (int j = 0; j < kSumsItems && i + j < t; ++j) {
+        const int m = c0 + i + j;
+        const long long hi = count_below(ws.segs, ns, s[j + 1]);
+        if (m == M - 1) {
+            *count_out = (uint32_t)hi;
+            if (hi > cap) atomicExch(status, TSDFL_ERR_CAPACITY);
         }
+        copy_rows(particles, m, lo, hi, cap, out, idx_out);
+        lo = hi;
     }
-}
-
-__global__ void set_flags_kernel(int* exact_ok, int* serial, int* err)
-{
-    chain_enter();
-    *exact_ok = 1;
-    *serial = 0;
-    *err = 0;
 }
 
 // SystematicResampler's loop (novel_resampling.h:41-72) literally, for the
@@ -2623,15 +2695,15 @@ __global__ void set_flags_kernel(int* exact_ok, int* serial, int* err)
 // one thread walks it over tiles of weights the block stages in shared memory,
 // writing every particle's count and exclusive offset; the copies are made in
 // parallel afterwards.  A draw that stops advancing or a count beyond 4M + 16
-// (the reference would never finish) stops the walk and sets *err.  Run by
-// resample_sums_kernel's block when *ws.serial is set (neither parallel form
-// applies).
+// (the reference would never finish) stops the walk and sets *err.  Run by one
+// block when *ws.serial is set (neither parallel form applies).
 __device__ void systematic_chain_block(const float* __restrict__ w, int stride, int M, float u0,
                                        uint32_t* __restrict__ cnt, uint32_t* __restrict__ off,
-                                       unsigned long long* total, int* err)
+                                       unsigned long long* total, int* err, unsigned char* buf)
 {
-    __shared__ float sw[kChainTile];
-    __shared__ uint32_t sc[kChainTile], so[kChainTile];
+    float* sw = reinterpret_cast<float*>(buf);
+    uint32_t* sc = reinterpret_cast<uint32_t*>(sw + kChainTile);
+    uint32_t* so = sc + kChainTile;
     __shared__ int s_stop;
     const double inv_m = 1.0 / (double)M;
     float u = u0;
@@ -2699,14 +2771,7 @@ __device__ void scatter_block(const float* particles, int M, const uint32_t* cnt
     }
     if (m >= M) return;
     const long long o = off[m];
-    for (long long j = o; j < o + (long long)cnt[m] && j < cap; ++j) {
-        if (idx_out) idx_out[j] = (uint32_t)m;
-        if (out) {
-            const float* src = particles + 7 * (size_t)m;
-            float* dst = out + 7 * (size_t)j;
-            for (int k = 0; k < 7; ++k) dst[k] = src[k];
-        }
-    }
+    copy_rows(particles, m, o, o + (long long)cnt[m], cap, out, idx_out);
 }
 
 // Best particle of mcl_3d.cpp:382-394: the first index with the largest weight
@@ -2802,15 +2867,16 @@ int check(cudaError_t e)
 // ------------------------------------------------------------------ launchers
 
 int launch_pose_prepare(const float* tf, const float* particles, int P, const float* points, int N, int npad,
-                        float max_range_sq, float c_in, float c_out, const float* code_values, int shift,
+                        float max_range_sq, float c_in, float c_out, const float* code_values, int shift, bool order,
                         const EvalBuffers& b, cudaStream_t s)
 {
     Tf16 t;
     for (int k = 0; k < 16; ++k) t.v[k] = tf[k];
+    const int groups = (P + kPoseSlots - 1) / kPoseSlots;   // a warp each
+    const int warps = std::max(1, std::min(kPoseThreads / 32, (groups + kPoseBlocks - 1) / kPoseBlocks));
     PointParams p{points, N, npad, 32 * ((N + 63) / 64), particles, P, max_range_sq, c_in, c_out, code_values,
-                  shift};
-    launch_chained(pose_prepare_kernel, (unsigned)(1 + pose_blocks((size_t)(P > 0 ? P : 0))), kPoseThreads, 0, s,
-                   t, p, b);
+                  shift, order ? 1 : 0, warps};
+    launch_chained(pose_prepare_kernel, (unsigned)(1 + (groups + warps - 1) / warps), kPoseThreads, 0, s, t, p, b);
     g_launches += 1;
     return check(cudaGetLastError());
 }
@@ -2965,7 +3031,7 @@ int launch_eval_pass(const MapView& m, float a_hit, int P, int n0, int n1, int n
         // the debug kernel scores either kind of cloud; otherwise the one of the
         // two kernels that the staging kernel's choice is not meant for returns at
         // once.  The spread one takes the whole scan, beside the first pass.
-        if (!dbg && first) {
+        if (!dbg && first && order_particles((size_t)P, (size_t)n_total)) {
             SpreadParams sp;
             sp.e = p;
             sp.work = b.work + 2;
@@ -3123,17 +3189,19 @@ int launch_norm(int P, int mode, int shift, double a_hit, double c_in, double c_
     const int nb = std::max(1, std::min(kNormBlocks, (P + kNormThreads - 1) / kNormThreads));
     NormParams q{P, mode, shift, a_hit, c_in, c_out, n_points, nin};
     launch_chained(norm_partial_kernel, (unsigned)nb, kNormThreads, 0, s, q, b, sum_f64);
-    launch_chained(norm_final_kernel, 1, kNormBlocks, 0, s, b, pose_out, nb);
-    g_launches += 2;
+    g_launches += 1;
     if (P > 0 && log_domain) {
+        launch_chained(norm_final_kernel, 1, kNormThreads, 0, s, b, pose_out, nb);
         cudaMemsetAsync(b.counts + 1, 0, sizeof(int32_t), s);
         log_max_kernel<<<kNormBlocks, kNormThreads, 0, s>>>(P, b);
         log_sum_kernel<<<kNormBlocks, kNormThreads, 0, s>>>(P, b);
         log_final_kernel<<<1, kNormBlocks, 0, s>>>(b);
         normalize_log_kernel<<<(P + 255) / 256, 256, 0, s>>>(P, b, particles_out, sticky);
-        g_launches += 4;
-    } else if (P > 0) {
-        launch_chained(normalize_kernel, (unsigned)((P + 255) / 256), 256, 0, s, P, b, particles_out, sticky);
+        g_launches += 5;
+    } else {
+        // at most a few blocks an SM: each adds the weight sum's partials once
+        const unsigned blocks = (unsigned)std::min((P + kNormThreads - 1) / kNormThreads, 4 * 148);
+        launch_chained(normalize_kernel, 1u + blocks, kNormThreads, 0, s, P, b, particles_out, pose_out, nb, sticky);
         g_launches += 1;
     }
     return check(cudaGetLastError());
@@ -3144,12 +3212,12 @@ size_t resample_workspace_bytes(size_t M)
     size_t tiles = (M + kScanTile - 1) / kScanTile + 1;
     size_t chunks = (M + kSumsChunk - 1) / kSumsChunk + 1;
     // flags: 16 + 16 + 8 + 4 + 4 <= 64
-    return 8 * (M + 3 * tiles) + sizeof(Segment) * kMaxSegments + 64 + sizeof(SumsChunk) * chunks;
+    return 8 * (M + 3 * tiles) + 4 * (tiles + 1) + sizeof(Segment) * kMaxSegments + 64 + sizeof(SumsChunk) * chunks;
 }
 
 int launch_resample_impl(const float* particles, const float* w, int stride, size_t M, float u0, float* out,
-                         uint32_t* idx_out, size_t cap, uint32_t* count_out, void* workspace, int32_t* status,
-                         cudaStream_t s, const float* u0p)
+                         uint32_t* idx_out, size_t cap, uint32_t* count_out, void* workspace, uint32_t* done,
+                         int32_t* status, cudaStream_t s, const float* u0p)
 {
     size_t tiles = (M + kScanTile - 1) / kScanTile;
     char* p = static_cast<char*>(workspace);
@@ -3159,33 +3227,30 @@ int launch_resample_impl(const float* particles, const float* w, int stride, siz
     ws.tile_off = reinterpret_cast<long long*>(p); p += 8 * (tiles + 1);
     ws.segs = reinterpret_cast<Segment*>(p); p += sizeof(Segment) * kMaxSegments;
     ws.nseg = reinterpret_cast<int*>(p); p += 16;
-    ws.exact_ok = reinterpret_cast<int*>(p); p += 16;
+    ws.exact_ok = reinterpret_cast<int*>(p);
+    ws.reach = reinterpret_cast<double*>(p + 8); p += 16;
     ws.total = reinterpret_cast<long long*>(p); p += 8;
-    int* err = reinterpret_cast<int*>(p); p += 4;
+    ws.err = reinterpret_cast<int*>(p); p += 4;
     ws.serial = reinterpret_cast<int*>(p); p += 4;
     ws.tile_dsum = reinterpret_cast<double*>(p); p += 8 * (tiles + 1);
-    ws.chunks = reinterpret_cast<SumsChunk*>(p);
+    const unsigned chunks = (unsigned)((M + kSumsChunk - 1) / kSumsChunk);
+    ws.chunks = reinterpret_cast<SumsChunk*>(p); p += sizeof(SumsChunk) * (chunks + 1);
+    ws.tile_flag = reinterpret_cast<int*>(p);
     ws.sums = reinterpret_cast<double*>(ws.cdf);
     ws.u0p = u0p;
-    const unsigned chunks = (unsigned)((M + kSumsChunk - 1) / kSumsChunk);
+    ws.done = done;
     // the literal loop reuses the prefix-sum array for counts and offsets
     uint32_t* cnt = reinterpret_cast<uint32_t*>(ws.cdf);
     uint32_t* off = cnt + M;
-    unsigned long long* total = reinterpret_cast<unsigned long long*>(ws.total);
-    const unsigned blocks = (unsigned)((M + 255) / 256);
-    launch_chained(set_flags_kernel, 1, 1, 0, s, ws.exact_ok, ws.serial, err);
-    launch_chained(resample_scan_kernel, (unsigned)tiles, kScanThreads, 0, s, w, stride, (int)M, ws);
-    launch_chained(resample_segments_kernel, 1, 32, 0, s, (int)M, u0, (int)tiles, ws);
-    launch_chained(resample_assign_kernel, blocks, 256, 0, s, particles, (int)M, out, idx_out, (long long)cap,
-                   count_out, ws, status);
-    // exact fallbacks: serial double sums + parallel assignment, else the literal loop
-    launch_chained(resample_chunk_transfer_kernel, chunks ? chunks : 1u, kSumsThreads, 0, s, w, stride, (int)M, ws);
-    launch_chained(resample_sums_kernel, 1, kSumsThreads, 0, s, w, stride, (int)M, u0, ws, cnt, off, total, err);
-    launch_chained(resample_chunk_write_kernel, chunks ? chunks : 1u, kSumsThreads, 0, s, w, stride, (int)M, ws);
-    launch_chained(resample_fallback_assign_kernel, blocks, 256, 0, s, particles, (int)M, out, idx_out,
-                   (long long)cap, count_out, ws, status, (const uint32_t*)cnt, (const uint32_t*)off,
-                   (const unsigned long long*)total, (const int*)err);
-    g_launches += 8;
+    const unsigned blocks = (unsigned)((M + kSumsThreads - 1) / kSumsThreads);
+    // small clouds' copies over more SMs
+    const int per = blocks >= 128u ? kSumsThreads : (blocks >= 32u ? 256 : 64);
+    launch_chained(resample_scan_kernel, (unsigned)tiles + 1u, kScanThreads, 0, s, w, stride, (int)M, u0, ws);
+    launch_chained(resample_assign_kernel, (unsigned)((M + per - 1) / per), kSumsThreads, 0, s, particles, w, stride,
+                   (int)M, u0, out, idx_out, (long long)cap, count_out, ws, cnt, off, status, per);
+    launch_chained(resample_finish_kernel, blocks, kSumsThreads, 0, s, particles, w, stride, (int)M, out, idx_out,
+                   (long long)cap, count_out, ws, (const uint32_t*)cnt, (const uint32_t*)off, status);
+    g_launches += 3;
     return check(cudaGetLastError());
 }
 

@@ -123,11 +123,11 @@ struct MapView {
 constexpr int kSentinels = 4;
 
 // pose_prepare_kernel: blocks of kPoseThreads; in the pose blocks three lanes
-// per particle, kPoseSlots particles a warp.
+// per particle, kPoseSlots particles a warp, spread over about kPoseBlocks
+// blocks before a block's warps all work.
 constexpr int kPoseThreads = 1024;
 constexpr int kPoseSlots = 10;
-constexpr int kPoseParticlesPerBlock = (kPoseThreads / 32) * kPoseSlots;
-inline size_t pose_blocks(size_t P) { return (P + kPoseParticlesPerBlock - 1) / kPoseParticlesPerBlock; }
+constexpr int kPoseBlocks = 150;
 constexpr uint32_t kHashEmpty = 0xffffffffu;
 
 #ifdef __CUDACC__
@@ -205,7 +205,25 @@ inline int fixed_shift(double max_value, double n)
     return std::min(40, std::min(sum, packed));
 }
 
+// EvalBuffers::work: [0, 1] the tiled kernel's item counter and CTAs done,
+// [2..4] the spread kernel's, [kWorkResample, + 1] the resampler's block counters
+// of a filter that has its own evaluation buffers.
 constexpr int kWorkWords = 8;
+constexpr int kWorkResample = 6;
+
+// Clouds with so many lookups (particles x points each) are put in spatial order
+// when they are spread over the map, and scored by the spread kernel; with fewer
+// the sort's three launches and the finer walk cost more than the order gives
+// (a step without / with it, us: building 1.36 GB, 20,000 x 2,048 449 / 466, 100,000 x
+// 512 656 / 533, 32,000 x 2,048 663 / 543; warehouse 269 MB, 32,000 x 2,048 356 / 369,
+// 64,000 x 2,048 645 / 601).  The subsampling kernel, which keeps its walk, gains
+// earlier (10,000 x 256 80 / 81, 30,000 x 256 155 / 148, 300,000 x 256 1,079 / 971).
+constexpr unsigned long long kOrderFrom = 3ull << 24;
+constexpr unsigned long long kOrderFromSub = 1ull << 22;
+inline bool order_particles(size_t P, size_t points, unsigned long long from = kOrderFrom)
+{
+    return (unsigned long long)P * (unsigned long long)points >= from;
+}
 
 // Kernel launchers (kernels.cu)
 struct EvalBuffers {
@@ -246,10 +264,10 @@ struct EvalBuffers {
 // 4 x 4 transform) beside the scan staging (pair layout in spatial order,
 // likelihood tables, per-point constants); also clears the scoring sums.
 int launch_pose_prepare(const float* tf, const float* particles, int P, const float* points, int N, int npad,
-                        float max_range_sq, float c_in, float c_out, const float* code_values, int shift,
+                        float max_range_sq, float c_in, float c_out, const float* code_values, int shift, bool order,
                         const EvalBuffers& b, cudaStream_t s);
-// Runs after launch_pose_prepare: orders the particles of a spread cloud by
-// cell (b.order); for a compact cloud its kernels return at once.
+// Runs after launch_pose_prepare (with order set): orders the particles of a
+// spread cloud by cell (b.order); for a compact cloud its kernels return at once.
 int launch_particle_order(const float* particles, int P, const EvalBuffers& b, cudaStream_t s);
 size_t eval_smem_bytes(bool serial, int n);
 // Scan points one pass of the tiled kernel stages (0: the kernel cannot hold
@@ -298,10 +316,11 @@ uint32_t build_batch_segs(const BatchSegSpec* specs, int nseg, int chunk, int gr
 int launch_eval_batch(const void* d_segs, const BatchKinds& kinds, uint32_t* counter, int32_t* status, int sm_count,
                       cudaStream_t s);
 size_t resample_workspace_bytes(size_t M);
-// u0p (optional): the draw read from device memory when the kernels run.
+// done: two counters that are 0 between launches; u0p (optional): the draw read
+// from device memory when the kernels run.
 int launch_resample_impl(const float* particles, const float* w, int stride, size_t M, float u0, float* out,
-                         uint32_t* idx_out, size_t cap, uint32_t* count_out, void* workspace, int32_t* status,
-                         cudaStream_t s, const float* u0p = nullptr);
+                         uint32_t* idx_out, size_t cap, uint32_t* count_out, void* workspace, uint32_t* done,
+                         int32_t* status, cudaStream_t s, const float* u0p = nullptr);
 // ResidualSystematicResampler on the device (residual.cu); workspace: residual_workspace_bytes(M).
 size_t residual_workspace_bytes(size_t M);
 int launch_resample_residual(const float* particles, const float* w, int stride, size_t M, float u0, float* out,
