@@ -251,7 +251,9 @@ int tsdfl_best_particle_device(tsdfl_ctx* ctx, const float* d_particles, size_t 
  * one TSDFEvaluator::evaluate + SystematicResampler::resample, as the single
  * calls above) updated together.  Their scoring runs in ONE persistent launch
  * over a (filter, pass, point chunk, particle group) work queue; preparation,
- * normalisation and resampling are per-filter launches in the same stream.
+ * normalisation and resampling are per-filter launches, side by side on streams
+ * of the batch forked from and joined to the context's (one after another when
+ * filters share a buffer that one of them writes).
  * The whole update can be captured once as a CUDA graph and replayed.  Every
  * filter's results are the same as its single-filter tsdfl_evaluate_device +
  * tsdfl_resample_systematic_device results (exact sums; same draws).  All

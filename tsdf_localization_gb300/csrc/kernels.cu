@@ -1457,107 +1457,117 @@ __global__ void __launch_bounds__(kSubThreads, 1) eval_subsample_kernel(SubParam
     }
 }
 
-// Work items per batch of the persistent multi-filter launch: the CTA's warps
-// take them one at a time from a shared counter, so uneven items even out
-// before the CTA's next barrier.
-constexpr int kBatchDepth = 8;
-constexpr int kBatchItems = kTiledWarps * kBatchDepth;
+// Work items per batch, the unit in which the persistent multi-filter launch's
+// work is reported and its grid is bounded.
+constexpr int kBatchItems = kTiledWarps * 8;
 
 struct BatchSeg {
     EvalParams e;
     int chunk, group, groups, items;
-    int dense, two;
-    uint32_t first_batch;
+    uint32_t first_item;   // of the segments of its kind one after another
+    uint32_t next;         // the next item to be taken; cleared before the launch
 };
+
+// Segment a CTA starts on: the one its share of the items begins in, so that the
+// CTAs spread over the segments by their work.  One warp; the same in every lane.
+__device__ __forceinline__ int batch_start(const BatchSeg* segs, int nseg, uint32_t total, int lane)
+{
+    const uint32_t at = (uint32_t)((unsigned long long)total * (2u * blockIdx.x + 1u) / (2u * gridDim.x));
+    int best = 0;
+    for (int k = lane; k < nseg; k += 32)
+        if (segs[k].first_item <= at) best = k;   // ascending
+    return __reduce_max_sync(0xffffffffu, best);
+}
+
+// Segment with the most items not taken yet, -1 when none has any.  One warp; the
+// same in every lane.
+__device__ __forceinline__ int batch_most_left(const BatchSeg* segs, int nseg, int lane)
+{
+    int left = 0, best = -1;
+    for (int k = lane; k < nseg; k += 32) {
+        const int v = segs[k].items - (int)min(*(const volatile uint32_t*)&segs[k].next, (uint32_t)segs[k].items);
+        if (v > left) {
+            left = v;
+            best = k;
+        }
+    }
+    const int most = __reduce_max_sync(0xffffffffu, left);
+    if (most == 0) return -1;
+    return __reduce_max_sync(0xffffffffu, left == most ? best : -1);
+}
 
 // Many filters in one persistent launch (one per map-layout kind present:
 // compact or brick table, one- or two-term sub-voxel multiplier -- the same
-// specialisations as eval_tiled_kernel).  The work queue is the filters'
-// (filter, pass) segments one after another, each cut into batches of
-// kBatchItems (point chunk, particle group) items.  A CTA takes the next batch
-// with one atomic, its warps take the batch's items from a shared counter;
-// when the batch belongs to another
-// segment than the one staged, the CTA stages that segment (the filter's code
-// LUT, its map's occupancy bitmap, the pass's scan points) before its warps
-// score the items.  Per-item scoring is eval_tiled_kernel's, so every filter's
-// sums equal its single-filter sums bit for bit.
+// specialisations as eval_tiled_kernel).  The work is the filters' (filter, pass)
+// segments, each of (point chunk, particle group) items that warps take from the
+// segment's own counter.  A CTA stages a segment (the filter's code LUT, its map's
+// occupancy bitmap, the pass's scan points), its warps score that segment's items
+// with no barrier between them until none is left, and the CTA goes on to the
+// segment with the most items left.  It begins where its share of all items
+// begins: most CTAs stage one segment and help out in one or two others at the
+// end.  (Batches of one queue, each taken by a CTA with barriers around it, put
+// all CTAs through every segment and left warps idle before each: see the figures
+// at the launch.)  Every item is taken once by the counter; a CTA leaves only
+// when no segment has an item left, so none is missed.  Per-item scoring is
+// eval_tiled_kernel's, so every filter's sums equal its single-filter sums bit for
+// bit.
 template <bool DENSE, bool TWO, bool MIN0>
-__global__ void __launch_bounds__(kTiledThreads, 1) eval_batch_kernel(const BatchSeg* __restrict__ segs, int nseg,
-                                                                      uint32_t total_batches, uint32_t* counter,
+__global__ void __launch_bounds__(kTiledThreads, 1) eval_batch_kernel(BatchSeg* segs, int nseg, uint32_t total_items,
                                                                       int32_t* status)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ uint64_t bar;
     __shared__ BatchSeg s_seg;
-    __shared__ uint32_t s_batch;
-    __shared__ uint32_t s_next;
     __shared__ int s_segi;
     LutEntry* lut = reinterpret_cast<LutEntry*>(smem);
     unsigned char* occ = smem + kLutTableBytes;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) mbar_init(&bar, 1);
+    if (warp == 0) {
+        const int k = batch_start(segs, nseg, total_items, lane);
+        if (lane == 0) s_segi = k;
+    }
     __syncthreads();
-    int cur = -1;
     uint32_t phase = 0;
-    float4* sxy = nullptr;
-    float2* spz = nullptr;
-    float4* ring = nullptr;
-    int n = 0;
     for (;;) {
-        if (threadIdx.x == 0) {
-            const uint32_t b = atomicAdd(counter, 1u);
-            int lo = 0, hi = nseg - 1;   // last segment whose first batch is <= b
-            while (lo < hi) {
-                const int mid = (lo + hi + 1) >> 1;
-                if (segs[mid].first_batch <= b) lo = mid;
-                else hi = mid - 1;
-            }
-            s_batch = b;
-            s_segi = lo;
-            s_next = 0;
-        }
-        __syncthreads();
-        const uint32_t b = s_batch;
         const int segi = s_segi;
-        if (b >= total_batches) break;
-        if (segi != cur) {
-            if (threadIdx.x == 0) s_seg = segs[segi];
-            __syncthreads();
-            const EvalParams& p = s_seg.e;
-            n = p.n1 - p.n0;
-            const int npairs = ((n + 63) >> 6) * 32;
-            const uint32_t occ_bytes = DENSE ? p.m.occ_bytes : 0u;
-            sxy = reinterpret_cast<float4*>(occ + occ_bytes);
-            spz = reinterpret_cast<float2*>(sxy + npairs);
-            ring = reinterpret_cast<float4*>(spz + npairs) + warp * kRing;
-            fill_lut(lut, p.lut_fx);
-            if (threadIdx.x == 0) {
-                mbar_expect_tx(&bar, (uint32_t)npairs * 24u + occ_bytes);
-                bulk_g2s(sxy, p.pxy + p.n0 / 2, (uint32_t)npairs * 16u, &bar);
-                bulk_g2s(spz, p.pz + p.n0 / 2, (uint32_t)npairs * 8u, &bar);
-                if (occ_bytes) bulk_g2s(occ, p.m.occ, occ_bytes, &bar);
-            }
-            bool staged = mbar_wait_bounded(&bar, phase);
-            if (!staged) staged = mbar_wait_bounded(&bar, phase);   // give copies in flight a second bound
-            phase ^= 1u;
-            if (!staged && threadIdx.x == 0) atomicExch(status, TSDFL_ERR_TIMEOUT);
-            if (__syncthreads_and(staged ? 1 : 0) == 0) return;
-            cur = segi;
+        if (segi < 0) break;
+        for (unsigned k = threadIdx.x; k < sizeof(BatchSeg) / 4u; k += kTiledThreads)
+            reinterpret_cast<uint32_t*>(&s_seg)[k] = reinterpret_cast<const uint32_t*>(segs + segi)[k];
+        __syncthreads();
+        const EvalParams& p = s_seg.e;
+        const int n = p.n1 - p.n0;
+        const int npairs = ((n + 63) >> 6) * 32;
+        const uint32_t occ_bytes = DENSE ? p.m.occ_bytes : 0u;
+        float4* sxy = reinterpret_cast<float4*>(occ + occ_bytes);
+        float2* spz = reinterpret_cast<float2*>(sxy + npairs);
+        float4* ring = reinterpret_cast<float4*>(spz + npairs) + warp * kRing;
+        fill_lut(lut, p.lut_fx);
+        if (threadIdx.x == 0) {
+            mbar_expect_tx(&bar, (uint32_t)npairs * 24u + occ_bytes);
+            bulk_g2s(sxy, p.pxy + p.n0 / 2, (uint32_t)npairs * 16u, &bar);
+            bulk_g2s(spz, p.pz + p.n0 / 2, (uint32_t)npairs * 8u, &bar);
+            if (occ_bytes) bulk_g2s(occ, p.m.occ, occ_bytes, &bar);
         }
-        const int base = (int)(b - s_seg.first_batch) * kBatchItems;
+        bool staged = mbar_wait_bounded(&bar, phase);
+        if (!staged) staged = mbar_wait_bounded(&bar, phase);   // give copies in flight a second bound
+        phase ^= 1u;
+        if (!staged && threadIdx.x == 0) atomicExch(status, TSDFL_ERR_TIMEOUT);
+        if (__syncthreads_and(staged ? 1 : 0) == 0) return;
         for (;;) {
-            uint32_t j = 0;
-            if (lane == 0) j = atomicAdd(&s_next, 1u);
-            j = __shfl_sync(0xffffffffu, j, 0);
-            const int item = base + (int)j;
-            if (j >= (uint32_t)kBatchItems || item >= s_seg.items) break;
-            const EvalParams& p = s_seg.e;
-            const int chunk = item / s_seg.groups, grp = item - chunk * s_seg.groups;
+            const uint32_t item = next_item(&segs[segi].next, lane);
+            if (item >= (uint32_t)s_seg.items) break;
+            const int chunk = (int)item / s_seg.groups, grp = (int)item - chunk * s_seg.groups;
             tiled_item<DENSE ? kLayBitmap : kLayTable, TWO, false, MIN0, true>(p, p.m, &p.m, occ, sxy, spz, lut, ring, n,
                                                                           s_seg.chunk, s_seg.group, chunk, grp,
                                                                           lane);
         }
-        __syncthreads();   // every warp is done with s_batch and the staged segment
+        __syncthreads();   // every warp is done with the staged segment
+        if (warp == 0) {
+            const int k = batch_most_left(segs, nseg, lane);
+            if (lane == 0) s_segi = k;
+        }
+        __syncthreads();
     }
 }
 
@@ -1724,6 +1734,11 @@ __device__ __forceinline__ void fold_status(const int32_t* ev, int32_t* sticky)
 {
     const int v = *ev;
     if (sticky && v && *sticky == 0) *sticky = v;
+}
+
+__global__ void fold_statuses_kernel(const int32_t* status, int n, int32_t* sticky)
+{
+    for (int i = 0; i < n && *sticky == 0; ++i) *sticky = status[i];
 }
 
 // particles[i].second = raw / weight_sum (tsdf_evaluator.cpp:203), skipped when
@@ -3114,10 +3129,10 @@ uint32_t build_batch_segs(const BatchSegSpec* specs, int nseg, int chunk, int gr
     });
     uint32_t total = 0;
     int o = 0;
-    for (int kind = 0; kind < 8; ++kind) {   // bit 2: min at the origin, bit 1: compact, bit 0: two-term
+    for (int kind = 0; kind < kBatchKinds; ++kind) {   // bit 2: min at the origin, bit 1: compact, bit 0: two-term
         kinds->first[kind] = o;
         kinds->count[kind] = 0;
-        uint32_t batches = 0;
+        uint32_t batches = 0, items = 0;
         for (int oi = 0; oi < nseg; ++oi) {
             const BatchSegSpec& sp = specs[order[oi]];
             const int k = (sp.m.min0 ? 4 : 0) + (sp.dense ? 2 : 0) + (sp.m.sub_fast == 1 ? 1 : 0);
@@ -3140,14 +3155,13 @@ uint32_t build_batch_segs(const BatchSegSpec* specs, int nseg, int chunk, int gr
             g.group = group;
             g.groups = (sp.P + group - 1) / group;
             g.items = ((sp.n1 - sp.n0 + chunk - 1) / chunk) * g.groups;
-            g.dense = sp.dense ? 1 : 0;
-            g.two = sp.m.sub_fast == 1 ? 1 : 0;
-            g.first_batch = batches;
+            g.first_item = items;
+            items += (uint32_t)g.items;
             batches += (uint32_t)((g.items + kBatchItems - 1) / kBatchItems);
             out[o++] = g;
             kinds->count[kind]++;
         }
-        kinds->batches[kind] = batches;
+        kinds->items[kind] = items;
         total += batches;
     }
     return total;
@@ -3155,26 +3169,33 @@ uint32_t build_batch_segs(const BatchSegSpec* specs, int nseg, int chunk, int gr
 
 size_t batch_smem_bytes() { return 227 * 1024 - 1024; }
 
-int launch_eval_batch(const void* d_segs, const BatchKinds& kinds, uint32_t* counter, int32_t* status,
-                      int sm_count, cudaStream_t s)
+// 24 filters (1,000-10,000 particles, 1,000-7,500 points, three maps), scoring and
+// all other kernels of an update: 2.36 ms with one queue of batches of 8 items a
+// warp and barriers around each, 1.94 with batches of 2 or 1, 1.75-1.78 with a
+// counter a segment and no barriers.  The kinds' launches follow one another: side by side on
+// streams of their own the update took 1.87 ms.
+int launch_eval_batch(void* d_segs, const BatchKinds& kinds, int32_t* status, int sm_count, cudaStream_t s)
 {
-    const BatchSeg* segs = static_cast<const BatchSeg*>(d_segs);
+    BatchSeg* segs = static_cast<BatchSeg*>(d_segs);
     const size_t smem = batch_smem_bytes();
-    using BatchKernel = void (*)(const BatchSeg*, int, uint32_t, uint32_t*, int32_t*);
-    static const BatchKernel kKinds[8] = {
+    using BatchKernel = void (*)(BatchSeg*, int, uint32_t, int32_t*);
+    static const BatchKernel kKinds[kBatchKinds] = {
         eval_batch_kernel<false, false, false>, eval_batch_kernel<false, true, false>,
         eval_batch_kernel<true, false, false>,  eval_batch_kernel<true, true, false>,
         eval_batch_kernel<false, false, true>,  eval_batch_kernel<false, true, true>,
         eval_batch_kernel<true, false, true>,   eval_batch_kernel<true, true, true>};
-    for (int kind = 0; kind < 8; ++kind) {
-        if (kinds.count[kind] == 0 || kinds.batches[kind] == 0) continue;
+    int nseg = 0;
+    for (int kind = 0; kind < kBatchKinds; ++kind) nseg += kinds.count[kind];
+    if (nseg == 0) return TSDFL_OK;
+    cudaMemset2DAsync(&segs->next, sizeof(BatchSeg), 0, sizeof(uint32_t), (size_t)nseg, s);   // the items' counters
+    for (int kind = 0; kind < kBatchKinds; ++kind) {
+        if (kinds.items[kind] == 0) continue;
         auto k = kKinds[kind];
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        cudaMemsetAsync(counter, 0, sizeof(uint32_t), s);
-        unsigned blocks = (unsigned)sm_count;
-        if (kinds.batches[kind] < blocks) blocks = kinds.batches[kind];
-        k<<<blocks, kTiledThreads, smem, s>>>(segs + kinds.first[kind], kinds.count[kind], kinds.batches[kind],
-                                              counter, status);
+        // no more CTAs than give every warp an item
+        const unsigned blocks =
+            std::min((unsigned)sm_count, (kinds.items[kind] + (unsigned)kTiledWarps - 1u) / (unsigned)kTiledWarps);
+        k<<<blocks, kTiledThreads, smem, s>>>(segs + kinds.first[kind], kinds.count[kind], kinds.items[kind], status);
         g_launches += 1;
     }
     return check(cudaGetLastError());
@@ -3204,6 +3225,13 @@ int launch_norm(int P, int mode, int shift, double a_hit, double c_in, double c_
         launch_chained(normalize_kernel, 1u + blocks, kNormThreads, 0, s, P, b, particles_out, pose_out, nb, sticky);
         g_launches += 1;
     }
+    return check(cudaGetLastError());
+}
+
+int launch_fold_status(const int32_t* status, int n, int32_t* sticky, cudaStream_t s)
+{
+    fold_statuses_kernel<<<1, 1, 0, s>>>(status, n, sticky);
+    g_launches += 1;
     return check(cudaGetLastError());
 }
 

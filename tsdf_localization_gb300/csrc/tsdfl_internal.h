@@ -303,9 +303,10 @@ struct BatchSegSpec {
 // The segments of each map-layout kind (bit 2: min corner at the origin, bit 1:
 // compact layout, bit 0: two-term sub-voxel multiplier) form one queue and one
 // persistent launch.
+constexpr int kBatchKinds = 8;
 struct BatchKinds {
-    int first[8], count[8];
-    uint32_t batches[8];
+    int first[kBatchKinds], count[kBatchKinds];
+    uint32_t items[kBatchKinds];
 };
 size_t batch_seg_bytes();
 // Writes nseg segment records (nseg * batch_seg_bytes() bytes at host_out),
@@ -313,8 +314,9 @@ size_t batch_seg_bytes();
 // returns the number of batches over all kinds.
 uint32_t build_batch_segs(const BatchSegSpec* specs, int nseg, int chunk, int group, void* host_out,
                           BatchKinds* kinds);
-int launch_eval_batch(const void* d_segs, const BatchKinds& kinds, uint32_t* counter, int32_t* status, int sm_count,
-                      cudaStream_t s);
+int launch_eval_batch(void* d_segs, const BatchKinds& kinds, int32_t* status, int sm_count, cudaStream_t s);
+// The first of n status words that is not 0 into *sticky, when that is still 0.
+int launch_fold_status(const int32_t* status, int n, int32_t* sticky, cudaStream_t s);
 size_t resample_workspace_bytes(size_t M);
 // done: two counters that are 0 between launches; u0p (optional): the draw read
 // from device memory when the kernels run.
