@@ -10,6 +10,7 @@
 
 #include "chain.h"
 #include "index_math.h"
+#include "pair_math.h"
 #include "subsample.h"
 #include "tsdfl_internal.h"
 
@@ -401,12 +402,20 @@ struct Tf16 {
     float v[16];
 };
 
+__device__ __noinline__ float2 sincos_double(float v)
+{
+    double s, c;
+    sincos((double)v, &s, &c);
+    return make_float2((float)s, (float)c);
+}
+
 // Laser pose of every particle (tsdf_evaluator.cpp:102-147): trig in double,
-// rounded to float (the correctly rounded sin/cos), products and sums in the
+// rounded to float (formed in float pairs; the double functions only where a pair
+// leaves the rounding open), products and sums in the
 // reference's order without contraction.  Three lanes per particle, ten
 // particles a warp (lanes 30 and 31 idle): lane 3p + k forms the sine and
 // cosine of angle k (roll, pitch, yaw), the three exchange them by shuffles,
-// and lane 3p + r forms row r of the 3 x 4 laser pose, so the FP64 latency of
+// and lane 3p + r forms row r of the 3 x 4 laser pose, so the latency of
 // the three sincos is spread over three lanes.  Also zeros in the scoring
 // sums, so no memset breaks the chain of kernels.  `blk` numbers the pose
 // blocks of pose_prepare_kernel; of each, `warps` warps work (a small cloud is
@@ -424,9 +433,13 @@ __device__ __forceinline__ void pose_block(int blk, int warps, const float* part
         hits[i] = 0;
     }
     const float* p = particles + 7 * (size_t)(active ? i : 0);
-    double sd, cd;
-    sincos((double)p[3 + (k < 3 ? k : 0)], &sd, &cd);
-    const float sv = (float)sd, cv = (float)cd;
+    const float angle = p[3 + (k < 3 ? k : 0)];
+    float sv, cv;
+    if (!sincos_rounded(angle, 0.0f, 0.0f, sv, cv)) {
+        const float2 v = sincos_double(angle);
+        sv = v.x;
+        cv = v.y;
+    }
     const int base = 3 * slot;
     auto from = [&](float v, int j) { return __shfl_sync(0xffffffffu, v, min(base + j, 31)); };
     const float sin_alpha = from(sv, 0), cos_alpha = from(cv, 0);
