@@ -851,8 +851,9 @@ constexpr int kTiledThreads = 736;
 constexpr int kTiledWarps = kTiledThreads / 32;
 constexpr int kSpreadThreads = 640;   // the spread kernel: registers before warps
 constexpr int kSpreadWarps = kSpreadThreads / 32;
-constexpr int kSubThreads = 768;      // the subsampling kernel, which waits on more gathers per lookup
+constexpr int kSubThreads = 1024;     // the subsampling kernel, which waits on more gathers per lookup
 constexpr int kSubWarps = kSubThreads / 32;
+constexpr size_t kSubSmem = 227 * 1024 - 1024;   // dynamic shared memory beside the static part
 constexpr int kRing = 64;   // deferred lookups per warp (transformed point + scan index)
 constexpr uint32_t kDbgSlow = 0x10000u;   // debug code flag: decided by the exact slow tiers
 
@@ -1350,20 +1351,27 @@ size_t spread_smem_bytes(uint32_t occ_bytes)
 
 // Seeded per-particle scan subsampling (subsample.h): one warp per particle
 // scores the particle's K kept points, two per lane per step, through the same
-// packed pipeline as the tiled kernel, reading the scan from the SoA arrays the
-// staging kernel wrote (scan order, L1-resident for scans of a few thousand
-// points).  Per particle: the fixed-point likelihood sum, the hits and the
-// number of kept points within max_range (its weight's range term), written
-// directly (one warp owns the particle).
+// packed pipeline as the tiled kernel.  Per particle: the fixed-point likelihood
+// sum, the hits and the number of kept points within max_range (its weight's
+// range term), written directly (one warp owns the particle).
+// Waits on the codes' gathers, so as many warps as the registers allow, and the
+// scan in shared memory where it fits (STAGED, one 16-byte read a point: four
+// reads from the SoA arrays took more of the L1's tag cycles than the gathers).
+// 300,000 particles x 256 of 2,048 points in the 100 x 100 m building, scoring: 850
+// us with two 64-bit divisions a point for its stratum and particles dealt to the
+// warps in turn; 726 with the strata stepped and particles from a counter; 676 with
+// 1,024 threads (768 before); 621 with the scan staged.
 struct SubParams {
     EvalParams e;
     int K;
     unsigned long long seed;
     uint32_t* nin;
     float c_in;
+    uint32_t* work;      // the item counter and the CTAs done
+    int group, items;    // particles an item, items
 };
 
-template <bool DENSE, bool TWO, bool MIN0>
+template <bool DENSE, bool TWO, bool MIN0, bool STAGED>
 __global__ void __launch_bounds__(kSubThreads, 1) eval_subsample_kernel(SubParams sp)
 {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -1375,8 +1383,12 @@ __global__ void __launch_bounds__(kSubThreads, 1) eval_subsample_kernel(SubParam
     const uint32_t occ_bytes = DENSE ? m.occ_bytes : 0u;
     unsigned char* occ = smem + kLutTableBytes;
     float4* rings = reinterpret_cast<float4*>(occ + occ_bytes);
+    float4* pts = rings + kRing * kSubWarps;
     if (threadIdx.x == 0) s_map = m;
     fill_lut(lut, p.lut_fx);
+    if (STAGED)
+        for (int j = threadIdx.x; j < p.n_total; j += kSubThreads)
+            pts[j] = make_float4(p.xs[j], p.ys[j], p.zs[j], p.cs[j]);
     if (threadIdx.x == 0) mbar_init(&bar, 1);
     __syncthreads();
     bool staged = true;
@@ -1395,23 +1407,55 @@ __global__ void __launch_bounds__(kSubThreads, 1) eval_subsample_kernel(SubParam
     float4* ring = rings + (threadIdx.x >> 5) * kRing;
     const PipeConsts K = pipe_consts(m);
     const uint32_t N = (uint32_t)p.n_total, Ks = (uint32_t)sp.K;
-    const int gwarp = blockIdx.x * kSubWarps + (threadIdx.x >> 5);
-    const int nwarps = gridDim.x * kSubWarps;
     const bool ordered = p.sched && *p.sched;
-    for (int q = gwarp; q < p.P; q += nwarps) {
+    // The strata's bounds floor(k N / K) of a lane's k = lane, lane + 64, ... (and
+    // lane + 32, ...), stepped with their remainders: exact, and no division a point.
+    const uint32_t qn = N / Ks, rn = N - qn * Ks;
+    const uint32_t q64 = (uint32_t)((64ull * N) / Ks), r64 = (uint32_t)(64ull * N - (uint64_t)q64 * Ks);
+    const uint32_t first_a = (uint32_t)(((uint64_t)lane * N) / Ks),
+                   first_b = (uint32_t)(((uint64_t)(lane + 32) * N) / Ks);
+    const uint32_t rem_a = (uint32_t)((uint64_t)lane * N - (uint64_t)first_a * Ks),
+                   rem_b = (uint32_t)((uint64_t)(lane + 32) * N - (uint64_t)first_b * Ks);
+    // the kept point of the stratum from b (k N = b K + rem)
+    auto kept = [&](uint64_t st, uint32_t b, uint32_t rem) {
+        const uint32_t n = qn + (rem + rn >= Ks ? 1u : 0u);
+        return b + __umulhi((uint32_t)(sub_mix64(st) >> 32), n);
+    };
+    int q = 0, q1 = 0;   // the item's particles
+    for (;; ++q) {
+        if (q == q1) {
+            const uint32_t item = next_item(sp.work, lane);
+            if (item >= (uint32_t)sp.items) break;
+            q = (int)item * sp.group;
+            q1 = min(q + sp.group, p.P);
+        }
         const int pi = ordered ? (int)p.order[q] : q;   // neighbouring warps take neighbouring particles
         const PosePairs R = pose_pairs(p.pose12 + 12 * (size_t)pi);
-        const uint64_t st = sub_particle_state(sp.seed, (uint64_t)pi);
+        uint64_t st_a = sub_particle_state(sp.seed, (uint64_t)pi) + (uint64_t)(lane + 1) * kGoldenGamma;
+        uint32_t b_a = first_a, m_a = rem_a, b_b = first_b, m_b = rem_b;
         long long acc = 0, sum = 0;
         uint32_t hits = 0, nin = 0, head = 0, tail = 0;
         int packed = 0;
         for (uint32_t base = 0; base < Ks; base += 64) {   // the same trip count on every lane
             const uint32_t ka = base + (uint32_t)lane, kb = ka + 32u;
             const bool va = ka < Ks, vb = kb < Ks;
-            const uint32_t ja = sub_point(st, N, Ks, va ? ka : 0u), jb = sub_point(st, N, Ks, vb ? kb : 0u);
-            const float xa = __ldg(p.xs + ja), ya = __ldg(p.ys + ja), za = __ldg(p.zs + ja);
-            const float xb = __ldg(p.xs + jb), yb = __ldg(p.ys + jb), zb = __ldg(p.zs + jb);
-            nin += (va && __ldg(p.cs + ja) == sp.c_in ? 1u : 0u) + (vb && __ldg(p.cs + jb) == sp.c_in ? 1u : 0u);
+            const uint32_t ja = va ? kept(st_a, b_a, m_a) : 0u;
+            const uint32_t jb = vb ? kept(st_a + 32u * kGoldenGamma, b_b, m_b) : 0u;
+            st_a += 64u * kGoldenGamma;
+            b_a += q64 + (m_a + r64 >= Ks ? 1u : 0u);
+            m_a = m_a + r64 >= Ks ? m_a + r64 - Ks : m_a + r64;
+            b_b += q64 + (m_b + r64 >= Ks ? 1u : 0u);
+            m_b = m_b + r64 >= Ks ? m_b + r64 - Ks : m_b + r64;
+            float4 A, B;
+            if (STAGED) {
+                A = pts[ja];
+                B = pts[jb];
+            } else {
+                A = make_float4(__ldg(p.xs + ja), __ldg(p.ys + ja), __ldg(p.zs + ja), __ldg(p.cs + ja));
+                B = make_float4(__ldg(p.xs + jb), __ldg(p.ys + jb), __ldg(p.zs + jb), __ldg(p.cs + jb));
+            }
+            const float xa = A.x, ya = A.y, za = A.z, xb = B.x, yb = B.y, zb = B.z;
+            nin += (va && A.w == sp.c_in ? 1u : 0u) + (vb && B.w == sp.c_in ? 1u : 0u);
             uint32_t k0, k1;
             bool s0, s1;
             pair_lookup<DENSE ? kLayBitmap : kLayTable, TWO, MIN0>(m, occ, R, K, pk(xa, xb), pk(ya, yb), pk(za, zb),
@@ -1468,6 +1512,7 @@ __global__ void __launch_bounds__(kSubThreads, 1) eval_subsample_kernel(SubParam
             sp.nin[pi] = nin;
         }
     }
+    items_done(sp.work);
 }
 
 // Work items per batch, the unit in which the persistent multi-filter launch's
@@ -3087,9 +3132,11 @@ int launch_eval_pass(const MapView& m, float a_hit, int P, int n0, int n1, int n
 }
 
 template <bool DENSE, bool TWO>
-void (*pick_sub_2(bool min0))(SubParams)
+void (*pick_sub_2(bool min0, bool staged))(SubParams)
 {
-    return min0 ? eval_subsample_kernel<DENSE, TWO, true> : eval_subsample_kernel<DENSE, TWO, false>;
+    if (staged)
+        return min0 ? eval_subsample_kernel<DENSE, TWO, true, true> : eval_subsample_kernel<DENSE, TWO, false, true>;
+    return min0 ? eval_subsample_kernel<DENSE, TWO, true, false> : eval_subsample_kernel<DENSE, TWO, false, false>;
 }
 
 int launch_eval_subsample(const MapView& m, float a_hit, int P, int N, int K, unsigned long long seed, float c_in,
@@ -3115,13 +3162,18 @@ int launch_eval_subsample(const MapView& m, float a_hit, int P, int N, int K, un
     sp.nin = b.nin;
     sp.c_in = c_in;
     const bool dense = m.occ_bytes != 0, two = m.sub_fast == 1;
-    auto k = dense ? (two ? pick_sub_2<true, true>(m.min0 != 0) : pick_sub_2<true, false>(m.min0 != 0))
-                   : (two ? pick_sub_2<false, true>(m.min0 != 0) : pick_sub_2<false, false>(m.min0 != 0));
-    const size_t smem = (size_t)kLutTableBytes + (dense ? (size_t)m.occ_bytes : 0) + sizeof(float4) * kRing * kSubWarps;
+    size_t smem = (size_t)kLutTableBytes + (dense ? (size_t)m.occ_bytes : 0) + sizeof(float4) * kRing * kSubWarps;
+    const bool staged = smem + sizeof(float4) * (size_t)N <= kSubSmem;
+    if (staged) smem += sizeof(float4) * (size_t)N;
+    auto k = dense ? (two ? pick_sub_2<true, true>(m.min0 != 0, staged) : pick_sub_2<true, false>(m.min0 != 0, staged))
+                   : (two ? pick_sub_2<false, true>(m.min0 != 0, staged) : pick_sub_2<false, false>(m.min0 != 0, staged));
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int blocks = sm_count;
     const int need = (P + kSubWarps - 1) / kSubWarps;
     if (need < blocks) blocks = need > 0 ? need : 1;
+    sp.work = b.work;
+    sp.group = P >= 32 * blocks * kSubWarps ? 2 : 1;   // 300,000 x 256: 711 us, 718 singly, 732 in fours
+    sp.items = (P + sp.group - 1) / sp.group;
     k<<<blocks, kSubThreads, smem, s>>>(sp);
     g_launches += 1;
     return check(cudaGetLastError());
