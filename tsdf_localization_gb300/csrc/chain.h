@@ -37,6 +37,27 @@ inline void launch_chained_2d(void (*kernel)(Params...), dim3 grid, unsigned blo
     cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+// The same with the grid in clusters of `cluster` blocks (of which grid is a multiple).
+template <typename... Params, typename... Args>
+inline void launch_chained_clusters(void (*kernel)(Params...), unsigned grid, unsigned cluster, unsigned block,
+                                    cudaStream_t s, Args... args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 template <typename... Params, typename... Args>
 inline void launch_chained(void (*kernel)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
                            Args... args)

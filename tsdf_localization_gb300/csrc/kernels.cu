@@ -1,11 +1,13 @@
 // Sensor-update kernels for sm_103a: pose build, scan staging, per-particle
 // scoring, normalisation / mean pose, systematic resampling, map re-layout.
+#include <cooperative_groups.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include <algorithm>
 #include <atomic>
+#include <utility>
 #include <vector>
 
 #include "chain.h"
@@ -15,6 +17,8 @@
 #include "tsdfl_internal.h"
 
 namespace tsdfl {
+
+namespace cg = cooperative_groups;
 
 std::atomic<unsigned long long> g_launches{0};
 
@@ -165,6 +169,7 @@ constexpr int kSortSectors = 16;
 constexpr int kSortBins = 2048;
 constexpr float kWideCloud = 10.0f;   // metres
 constexpr int kPrepThreads = 1024;
+constexpr int kPrepBlocks = 8;      // one cluster
 constexpr int kBinCache = 16384;    // points whose bin the staging keeps in shared memory
 static_assert(kSortBins == 2 * kPrepThreads, "two bins per thread in the scan");
 
@@ -188,22 +193,33 @@ __device__ __forceinline__ int spatial_bin(float x, float y, float z, bool wide)
 // score constant of tsdf_evaluator.cpp:56-65 and the number of points inside
 // max_range; the pair layout of the tiled kernels in spatial order (a counting
 // sort by spatial_bin; perm records each position's scan index); also the
-// likelihood tables for this scan.  Block 0 of pose_prepare_kernel, beside the
-// pose blocks.  Which order suits the cloud (compact or spread) is decided on
+// likelihood tables for this scan.  The first cluster of pose_prepare_kernel, beside
+// the pose blocks: each of its kPrepBlocks blocks counts and places a slice of the
+// scan, and reads the others' counts from their shared memory.  Bound by the
+// scattered 4-byte stores of the pair layout, one tag a lane, so one block took
+// 29 us for 16,384 points and 11 for 2,048 (a cloud update of 2,000 particles 230 us
+// a pass, 219 with the cluster; an update and resampling of 1,000 x 2,048 55.9 and
+// 54.1).  Which order suits the cloud (compact or spread) is decided on
 // the x / y extent of a sample of at most kExtentSample particles, and the
 // particle order's cells span that extent (clamped at its edges); both only
 // decide how fast the scoring runs, never what it returns.
 constexpr int kExtentSample = 4096;
 
-__device__ __forceinline__ void prepare_points_block(const PointParams& p, const EvalBuffers& b)
+__device__ __forceinline__ void prepare_points_block(const PointParams& p, const EvalBuffers& b, int rank)
 {
     __shared__ int warp_counts[32];
-    __shared__ int bins[kSortBins];
+    __shared__ int2 bins[kPrepThreads];      // this slice's points a bin, two bins a thread
+    __shared__ int places[kSortBins];        // the next position of a bin's points of this slice
     __shared__ uint16_t sbin[kBinCache];
     __shared__ float4 s_ext[32];
-    __shared__ int s_wide;
-    if (threadIdx.x == 0) *b.status = 0;
-    if (p.order)
+    __shared__ int s_wide, s_in;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int slice = ((p.npad + kPrepBlocks - 1) / kPrepBlocks + 31) & ~31;
+    const int j0 = (int)min((long long)rank * slice, (long long)p.npad);
+    const int jpad = min(p.npad - j0, slice) + j0, j1 = min(jpad, p.N);
+    if (rank == 0 && threadIdx.x == 0) *b.status = 0;
+    if (rank == 0 && p.order)
         for (int c = threadIdx.x; c < kCellBins; c += blockDim.x) b.phist[c] = 0;   // the particle order's histogram
     {   // the cloud's x / y extent from a sample of the particles
         const float inf = __int_as_float(0x7f800000);
@@ -215,25 +231,24 @@ __device__ __forceinline__ void prepare_points_block(const PointParams& p, const
             e = make_float4(fminf(e.x, x), fminf(e.y, y), fmaxf(e.z, x), fmaxf(e.w, y));
         }
         e = warp_extent(e);
-        if ((threadIdx.x & 31) == 0) s_ext[threadIdx.x >> 5] = e;
+        if (lane == 0) s_ext[warp] = e;
+        if (threadIdx.x == 0) s_in = 0;
         __syncthreads();
+        if (warp == 0) e = warp_extent(s_ext[lane]);
         if (threadIdx.x == 0) {
-            for (int w = 1; w < (int)(blockDim.x >> 5); ++w) {
-                const float4 v = s_ext[w];
-                e = make_float4(fminf(e.x, v.x), fminf(e.y, v.y), fmaxf(e.z, v.z), fmaxf(e.w, v.w));
-            }
             s_wide = fmaxf(e.z - e.x, e.w - e.y) > kWideCloud ? 1 : 0;   // no particles: -inf
-            b.counts[2] = p.order ? s_wide : 0;   // the particles are put in spatial order too
-            for (int k = 0; k < kWorkWords; ++k) b.work[k] = 0u;
-            b.cloud_ext[0] = e;
+            if (rank == 0) {
+                b.counts[2] = p.order ? s_wide : 0;   // the particles are put in spatial order too
+                for (int k = 0; k < kWorkWords; ++k) b.work[k] = 0u;
+                b.cloud_ext[0] = e;
+            }
         }
     }
-    for (int i = threadIdx.x; i < kSortBins; i += blockDim.x) bins[i] = 0;
+    bins[threadIdx.x] = make_int2(0, 0);
     __syncthreads();
     const bool wide = s_wide != 0;
     int in = 0;
-#pragma unroll 4
-    for (int j = threadIdx.x; j < p.npad; j += blockDim.x) {
+    for (int j = j0 + (int)threadIdx.x; j < jpad; j += blockDim.x) {
         float x = 0, y = 0, z = 0, c = 0;
         if (j < p.N) {
             x = __ldg(p.points + 3 * j);
@@ -244,18 +259,32 @@ __device__ __forceinline__ void prepare_points_block(const PointParams& p, const
             c = inr ? p.c_in : p.c_out;
             in += inr ? 1 : 0;
             const int bin = spatial_bin(x, y, z, wide);
-            atomicAdd(&bins[bin], 1);
-            if (j < kBinCache) sbin[j] = (uint16_t)bin;
+            atomicAdd(&reinterpret_cast<int*>(bins)[bin], 1);
+            if (j - j0 < kBinCache) sbin[j - j0] = (uint16_t)bin;
         }
         ((float*)b.xs)[j] = x;
         ((float*)b.ys)[j] = y;
         ((float*)b.zs)[j] = z;
         ((float*)b.cs)[j] = c;
     }
-    __syncthreads();   // counts complete; this block's SoA stores visible to it
-    {   // exclusive scan of the bin counts, two bins per thread
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        const int c0 = bins[2 * threadIdx.x], c1 = bins[2 * threadIdx.x + 1];
+    in = (int)warp_sum_u32((uint32_t)in);
+    if (lane == 0 && in) atomicAdd(&s_in, in);
+    cluster.sync();   // every slice's counts are complete
+    {   // exclusive scan of the bins' counts, and within a bin of the slices'
+        int c0 = 0, c1 = 0, b0 = 0, b1 = 0, n_in = 0;
+#pragma unroll
+        for (int r = 0; r < kPrepBlocks; ++r) {
+            const int2 c = *cluster.map_shared_rank(&bins[threadIdx.x], r);
+            b0 += r < rank ? c.x : 0;
+            b1 += r < rank ? c.y : 0;
+            c0 += c.x;
+            c1 += c.y;
+        }
+        if (rank == 0 && threadIdx.x < kPrepBlocks) n_in = *cluster.map_shared_rank(&s_in, threadIdx.x);
+        if (rank == 0 && warp == 0) {
+            n_in = (int)warp_sum_u32((uint32_t)n_in);
+            if (lane == 0) b.counts[0] = n_in;
+        }
         int v = c0 + c1;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -265,7 +294,7 @@ __device__ __forceinline__ void prepare_points_block(const PointParams& p, const
         if (lane == 31) warp_counts[warp] = v;
         __syncthreads();
         if (warp == 0) {
-            int w = lane < (int)(blockDim.x >> 5) ? warp_counts[lane] : 0;
+            int w = warp_counts[lane];
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const int t = __shfl_up_sync(0xffffffffu, w, o);
@@ -275,15 +304,16 @@ __device__ __forceinline__ void prepare_points_block(const PointParams& p, const
         }
         __syncthreads();
         const int before = (warp ? warp_counts[warp - 1] : 0) + v - c0 - c1;
-        bins[2 * threadIdx.x] = before;
-        bins[2 * threadIdx.x + 1] = before + c0;
+        places[2 * threadIdx.x] = before + b0;
+        places[2 * threadIdx.x + 1] = before + c0 + b1;
     }
     __syncthreads();
+    cg::cluster_group::arrival_token done = cluster.barrier_arrive();   // the other blocks' memory has been read
     // pair layout of the fast kernel: in every block of 64 positions, lane l of
     // a warp takes positions 64*blk + l and 64*blk + 32 + l
-    for (int j = threadIdx.x; j < p.N; j += blockDim.x) {
-        const float x = b.xs[j], y = b.ys[j], z = b.zs[j];
-        const int q = atomicAdd(&bins[j < kBinCache ? (int)sbin[j] : spatial_bin(x, y, z, wide)], 1);
+    for (int j = j0 + (int)threadIdx.x; j < j1; j += blockDim.x) {
+        const float x = __ldg(p.points + 3 * j), y = __ldg(p.points + 3 * j + 1), z = __ldg(p.points + 3 * j + 2);
+        const int q = atomicAdd(&places[j - j0 < kBinCache ? (int)sbin[j - j0] : spatial_bin(x, y, z, wide)], 1);
         const int pair = (q >> 6) * 32 + (q & 31), half = (q >> 5) & 1;
         float* xy = reinterpret_cast<float*>(b.pxy + pair);
         xy[half] = x;
@@ -291,7 +321,8 @@ __device__ __forceinline__ void prepare_points_block(const PointParams& p, const
         reinterpret_cast<float*>(b.pz + pair)[half] = z;
         b.perm[q] = j;
     }
-    for (int q = p.N + threadIdx.x; q < 2 * p.npairs; q += blockDim.x) {   // padding positions
+    const int at = rank * (int)blockDim.x + (int)threadIdx.x, step = kPrepBlocks * (int)blockDim.x;
+    for (int q = p.N + at; q < 2 * p.npairs; q += step) {   // padding positions
         const int pair = (q >> 6) * 32 + (q & 31), half = (q >> 5) & 1;
         float* xy = reinterpret_cast<float*>(b.pxy + pair);
         xy[half] = 0.0f;
@@ -299,19 +330,13 @@ __device__ __forceinline__ void prepare_points_block(const PointParams& p, const
         reinterpret_cast<float*>(b.pz + pair)[half] = 0.0f;
         b.perm[q] = 0;   // never read: padding lanes record no debug code
     }
-    for (int c = threadIdx.x; c < kNumCodes; c += blockDim.x) {
-        float v = p.code_values[c];
-        b.lut_f[c] = v;
-        b.lut_fx[c] = __double2ll_rn(ldexp((double)v, p.shift));
-    }
-    in = (int)warp_sum_u32((uint32_t)in);
-    if ((threadIdx.x & 31) == 0) warp_counts[threadIdx.x >> 5] = in;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int t = 0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += warp_counts[w];
-        b.counts[0] = t;
-    }
+    if (rank == kPrepBlocks - 1)
+        for (int c = threadIdx.x; c < kNumCodes; c += blockDim.x) {
+            float v = p.code_values[c];
+            b.lut_f[c] = v;
+            b.lut_fx[c] = __double2ll_rn(ldexp((double)v, p.shift));
+        }
+    cluster.barrier_wait(std::move(done));   // no block leaves while its counts may be read
 }
 
 // Spatial order of a spread cloud's particles (global localisation): 64 x 64
@@ -475,14 +500,14 @@ __device__ __forceinline__ void pose_block(int blk, int warps, const float* part
     tg[2 * k + 1] = cv;
 }
 
-// First kernel of an update: block 0 stages the scan (prepare_points_block),
-// the others form the laser poses (pose_block); the two parts share no data,
-// so they run side by side.
+// First kernel of an update, in clusters of kPrepBlocks: the first cluster stages the
+// scan (prepare_points_block), the others form the laser poses (pose_block); the two
+// parts share no data, so they run side by side.
 __global__ void __launch_bounds__(kPoseThreads) pose_prepare_kernel(Tf16 tf, PointParams p, EvalBuffers b)
 {
     chain_enter();
-    if (blockIdx.x == 0) prepare_points_block(p, b);
-    else pose_block((int)blockIdx.x - 1, p.pose_warps, p.particles, p.P, tf, b.pose12, b.trig6, b.sum_fx, b.hits);
+    if (blockIdx.x < kPrepBlocks) prepare_points_block(p, b, (int)blockIdx.x);
+    else pose_block((int)blockIdx.x - kPrepBlocks, p.pose_warps, p.particles, p.P, tf, b.pose12, b.trig6, b.sum_fx, b.hits);
 }
 
 struct EvalParams {
@@ -851,8 +876,12 @@ constexpr int kTiledThreads = 736;
 constexpr int kTiledWarps = kTiledThreads / 32;
 constexpr int kSpreadThreads = 640;   // the spread kernel: registers before warps
 constexpr int kSpreadWarps = kSpreadThreads / 32;
-constexpr int kSubThreads = 1024;     // the subsampling kernel, which waits on more gathers per lookup
-constexpr int kSubWarps = kSubThreads / 32;
+// The subsampling kernel, which waits on more gathers per lookup, so 1,024 threads;
+// with a bitmap in shared memory their rings leave the L1 too little for the codes
+// of neighbouring particles (150,000 x 200 of 4,096 points, warehouse, us: brick table
+// 338 with 1,024 threads, 394 with 768, compact layout 515 and 427; 150,000 x 200 of 2,048,
+// building, compact: 374 to 464 from one process to the next, and 416).
+__host__ __device__ constexpr int sub_threads(bool dense) { return dense ? 768 : 1024; }
 constexpr size_t kSubSmem = 227 * 1024 - 1024;   // dynamic shared memory beside the static part
 constexpr int kRing = 64;   // deferred lookups per warp (transformed point + scan index)
 constexpr uint32_t kDbgSlow = 0x10000u;   // debug code flag: decided by the exact slow tiers
@@ -1354,13 +1383,11 @@ size_t spread_smem_bytes(uint32_t occ_bytes)
 // packed pipeline as the tiled kernel.  Per particle: the fixed-point likelihood
 // sum, the hits and the number of kept points within max_range (its weight's
 // range term), written directly (one warp owns the particle).
-// Waits on the codes' gathers, so as many warps as the registers allow, and the
-// scan in shared memory where it fits (STAGED, one 16-byte read a point: four
-// reads from the SoA arrays took more of the L1's tag cycles than the gathers).
-// 300,000 particles x 256 of 2,048 points in the 100 x 100 m building, scoring: 850
-// us with two 64-bit divisions a point for its stratum and particles dealt to the
-// warps in turn; 726 with the strata stepped and particles from a counter; 676 with
-// 1,024 threads (768 before); 621 with the scan staged.
+// Waits on the codes' gathers.  300,000 particles x 256 of 2,048 points in the
+// 100 x 100 m building, compact layout, a pass: 1,018 us with two 64-bit divisions a
+// point for its stratum and particles dealt to the warps in turn; 815 with the
+// strata stepped and particles from a counter.  STAGED: the scan in shared memory,
+// one 16-byte read a point instead of four from the SoA arrays.
 struct SubParams {
     EvalParams e;
     int K;
@@ -1372,7 +1399,7 @@ struct SubParams {
 };
 
 template <bool DENSE, bool TWO, bool MIN0, bool STAGED>
-__global__ void __launch_bounds__(kSubThreads, 1) eval_subsample_kernel(SubParams sp)
+__global__ void __launch_bounds__(sub_threads(DENSE), 1) eval_subsample_kernel(SubParams sp)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ uint64_t bar;
@@ -1383,11 +1410,11 @@ __global__ void __launch_bounds__(kSubThreads, 1) eval_subsample_kernel(SubParam
     const uint32_t occ_bytes = DENSE ? m.occ_bytes : 0u;
     unsigned char* occ = smem + kLutTableBytes;
     float4* rings = reinterpret_cast<float4*>(occ + occ_bytes);
-    float4* pts = rings + kRing * kSubWarps;
+    float4* pts = rings + kRing * (sub_threads(DENSE) / 32);
     if (threadIdx.x == 0) s_map = m;
     fill_lut(lut, p.lut_fx);
     if (STAGED)
-        for (int j = threadIdx.x; j < p.n_total; j += kSubThreads)
+        for (int j = threadIdx.x; j < p.n_total; j += sub_threads(DENSE))
             pts[j] = make_float4(p.xs[j], p.ys[j], p.zs[j], p.cs[j]);
     if (threadIdx.x == 0) mbar_init(&bar, 1);
     __syncthreads();
@@ -2949,7 +2976,8 @@ int launch_pose_prepare(const float* tf, const float* particles, int P, const fl
     const int warps = std::max(1, std::min(kPoseThreads / 32, (groups + kPoseBlocks - 1) / kPoseBlocks));
     PointParams p{points, N, npad, 32 * ((N + 63) / 64), particles, P, max_range_sq, c_in, c_out, code_values,
                   shift, order ? 1 : 0, warps};
-    launch_chained(pose_prepare_kernel, (unsigned)(1 + (groups + warps - 1) / warps), kPoseThreads, 0, s, t, p, b);
+    const unsigned blocks = (unsigned)((groups + warps - 1) / warps + kPrepBlocks - 1) / kPrepBlocks * kPrepBlocks;
+    launch_chained_clusters(pose_prepare_kernel, kPrepBlocks + blocks, kPrepBlocks, kPoseThreads, s, t, p, b);
     g_launches += 1;
     return check(cudaGetLastError());
 }
@@ -3131,12 +3159,10 @@ int launch_eval_pass(const MapView& m, float a_hit, int P, int n0, int n1, int n
     return check(cudaGetLastError());
 }
 
-template <bool DENSE, bool TWO>
-void (*pick_sub_2(bool min0, bool staged))(SubParams)
+template <bool DENSE, bool TWO, bool STAGED>
+void (*pick_sub_2(bool min0))(SubParams)
 {
-    if (staged)
-        return min0 ? eval_subsample_kernel<DENSE, TWO, true, true> : eval_subsample_kernel<DENSE, TWO, false, true>;
-    return min0 ? eval_subsample_kernel<DENSE, TWO, true, false> : eval_subsample_kernel<DENSE, TWO, false, false>;
+    return min0 ? eval_subsample_kernel<DENSE, TWO, true, STAGED> : eval_subsample_kernel<DENSE, TWO, false, STAGED>;
 }
 
 int launch_eval_subsample(const MapView& m, float a_hit, int P, int N, int K, unsigned long long seed, float c_in,
@@ -3162,19 +3188,23 @@ int launch_eval_subsample(const MapView& m, float a_hit, int P, int N, int K, un
     sp.nin = b.nin;
     sp.c_in = c_in;
     const bool dense = m.occ_bytes != 0, two = m.sub_fast == 1;
-    size_t smem = (size_t)kLutTableBytes + (dense ? (size_t)m.occ_bytes : 0) + sizeof(float4) * kRing * kSubWarps;
-    const bool staged = smem + sizeof(float4) * (size_t)N <= kSubSmem;
+    const int threads = sub_threads(dense), warps_cta = threads / 32;
+    size_t smem = (size_t)kLutTableBytes + (dense ? (size_t)m.occ_bytes : 0) + sizeof(float4) * kRing * warps_cta;
+    // the scan beside no bitmap, where it fits: 150,000 x 200 of 5,500 points, warehouse,
+    // brick table 329 us, 348 from the SoA arrays
+    const bool staged = !dense && smem + sizeof(float4) * (size_t)N <= kSubSmem;
     if (staged) smem += sizeof(float4) * (size_t)N;
-    auto k = dense ? (two ? pick_sub_2<true, true>(m.min0 != 0, staged) : pick_sub_2<true, false>(m.min0 != 0, staged))
-                   : (two ? pick_sub_2<false, true>(m.min0 != 0, staged) : pick_sub_2<false, false>(m.min0 != 0, staged));
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    auto k = dense    ? (two ? pick_sub_2<true, true, false>(m.min0 != 0) : pick_sub_2<true, false, false>(m.min0 != 0))
+             : staged ? (two ? pick_sub_2<false, true, true>(m.min0 != 0) : pick_sub_2<false, false, true>(m.min0 != 0))
+                      : (two ? pick_sub_2<false, true, false>(m.min0 != 0) : pick_sub_2<false, false, false>(m.min0 != 0));
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSubSmem);
     int blocks = sm_count;
-    const int need = (P + kSubWarps - 1) / kSubWarps;
+    const int need = (P + warps_cta - 1) / warps_cta;
     if (need < blocks) blocks = need > 0 ? need : 1;
     sp.work = b.work;
-    sp.group = P >= 32 * blocks * kSubWarps ? 2 : 1;   // 300,000 x 256: 711 us, 718 singly, 732 in fours
+    sp.group = P >= 32 * blocks * warps_cta ? 2 : 1;   // 300,000 x 256 (1,024 threads): 711 us, 718 singly, 732 in fours
     sp.items = (P + sp.group - 1) / sp.group;
-    k<<<blocks, kSubThreads, smem, s>>>(sp);
+    k<<<blocks, threads, smem, s>>>(sp);
     g_launches += 1;
     return check(cudaGetLastError());
 }
