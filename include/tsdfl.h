@@ -232,8 +232,8 @@ int tsdfl_resample_systematic_device(tsdfl_ctx* ctx, const float* d_particles, s
  * default resampler (mcl_3d.cpp:765), with its draw u0 in [0, 1) given:
  * particle m is emitted (size_t)(temp + 1.0) times, temp = (float)M * w_m - u,
  * u then becomes (float)count - temp.  Bit-exact with the reference for the
- * same weights and u0 (the float chain is walked in particle order by one
- * device thread; the copies are parallel).  Negative or non-finite weights, or
+ * same weights and u0 (large clouds walk the float chain's likely starts in
+ * parallel, small ones one thread walks it).  Negative or non-finite weights, or
  * a particle count of 2^24, give TSDFL_ERR_UNSUPPORTED. */
 int tsdfl_resample_residual_systematic(tsdfl_ctx* ctx, const float* weights, size_t M, float u0, uint32_t* idx_out,
                                        size_t cap, size_t* count_out);
