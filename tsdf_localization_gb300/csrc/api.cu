@@ -153,7 +153,7 @@ size_t eval_layout(size_t nP, size_t nN, char* base, EvalBuffers* e, double** su
     size_t o_st = take(sizeof(int32_t) * 4);
     size_t o_ord = take(sizeof(uint32_t) * nP);
     size_t o_pk = take(sizeof(uint32_t) * nP);
-    size_t o_ph = take(sizeof(int32_t) * 4096);
+    size_t o_ph = take(sizeof(int32_t) * kCellBins);
     size_t o_ce = take(sizeof(float) * 4);
     if (base) {
         char* b = base;
@@ -1589,13 +1589,17 @@ int batch_score(tsdfl_batch* B, cudaStream_t s)
     return TSDFL_OK;
 }
 
-// Clears every filter's sums for another batch_score of the same poses.
+// Clears every filter's sums, and the cell histogram of those that batch_score
+// puts in spatial order, for another batch_score of the same poses.
 int batch_clear(tsdfl_batch* B, cudaStream_t s)
 {
     for (size_t i = 0; i < B->f.size(); ++i) {
-        if (!B->per[i].tiled || B->f[i].N == 0) continue;
-        CUDA_TRY(cudaMemsetAsync(B->per[i].b.sum_fx, 0, sizeof(long long) * B->f[i].P, s));
-        CUDA_TRY(cudaMemsetAsync(B->per[i].b.hits, 0, sizeof(uint32_t) * B->f[i].P, s));
+        const tsdfl_filter& F = B->f[i];
+        const tsdfl_batch::Per& q = B->per[i];
+        if (!q.tiled || F.N == 0) continue;
+        CUDA_TRY(cudaMemsetAsync(q.b.sum_fx, 0, sizeof(long long) * F.P, s));
+        CUDA_TRY(cudaMemsetAsync(q.b.hits, 0, sizeof(uint32_t) * F.P, s));
+        if (q.big && order_particles(F.P, F.N)) CUDA_TRY(cudaMemsetAsync(q.b.phist, 0, sizeof(int32_t) * kCellBins, s));
     }
     return TSDFL_OK;
 }

@@ -139,10 +139,6 @@ __device__ __forceinline__ uint32_t dense_code(const MapView& m, float x, float 
     return idx == kMissIndex ? (uint32_t)kCodeMiss : (uint32_t)__ldg(m.codes + idx);
 }
 
-// Spread clouds' particle order: 2^kCellBits x 2^kCellBits cells (below).
-constexpr int kCellBits = 6;
-constexpr int kCellBins = 1 << (2 * kCellBits);
-
 struct PointParams {
     const float* points;  // N x 3
     int N, npad, npairs;
@@ -2985,7 +2981,8 @@ int launch_pose_prepare(const float* tf, const float* particles, int P, const fl
 int launch_particle_order(const float* particles, int P, const EvalBuffers& b, cudaStream_t s)
 {
     if (P <= 0) return TSDFL_OK;
-    // the cell histogram was cleared by pose_prepare_kernel
+    // the cell histogram was cleared by pose_prepare_kernel (or, for another order of the
+    // same poses, by the caller): the scatter leaves the cells' ends in it
     const unsigned blocks = (unsigned)std::min((P + 255) / 256, 4096);
     launch_chained(particle_cells_kernel, blocks, 256, 0, s, particles, P, b);
     launch_chained(particle_scan_kernel, 1, kCellScanThreads, 0, s, b);

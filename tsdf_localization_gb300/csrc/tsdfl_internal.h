@@ -230,6 +230,10 @@ inline bool order_particles(size_t P, size_t points, unsigned long long from = k
     return lookups >= from || (P >= kOrderParticles && lookups >= kOrderManyFrom);
 }
 
+// Cells of the particle order (particle_cells_kernel): 2^kCellBits on a side.
+constexpr int kCellBits = 6;
+constexpr int kCellBins = 1 << (2 * kCellBits);
+
 // Kernel launchers (kernels.cu)
 struct EvalBuffers {
     const float* particles;  // P x 7
@@ -261,7 +265,7 @@ struct EvalBuffers {
     // cells over the cloud's x / y extent (cloud_ext).
     uint32_t* order;         // P
     uint32_t* pkeys;         // P: each particle's cell
-    int32_t* phist;          // kCellBins: cell counts, then offsets
+    int32_t* phist;          // kCellBins: cell counts, then the cells' ends; 0 before an order
     float4* cloud_ext;       // [1]: min x, min y, max x, max y of the particles
 };
 
@@ -271,8 +275,9 @@ struct EvalBuffers {
 int launch_pose_prepare(const float* tf, const float* particles, int P, const float* points, int N, int npad,
                         float max_range_sq, float c_in, float c_out, const float* code_values, int shift, bool order,
                         const EvalBuffers& b, cudaStream_t s);
-// Runs after launch_pose_prepare (with order set): orders the particles of a
-// spread cloud by cell (b.order); for a compact cloud its kernels return at once.
+// Runs after launch_pose_prepare (with order set), and again only after a clear of
+// b.phist: orders the particles of a spread cloud by cell (b.order); for a compact
+// cloud its kernels return at once.
 int launch_particle_order(const float* particles, int P, const EvalBuffers& b, cudaStream_t s);
 size_t eval_smem_bytes(bool serial, int n);
 // Scan points one pass of the tiled kernel stages (0: the kernel cannot hold
