@@ -26,6 +26,7 @@ namespace {
 
 constexpr int kLutBytes = ((kNumCodes * 8 + 15) / 16) * 16;
 constexpr int kLutFBytes = ((kNumCodes * 4 + 15) / 16) * 16;
+static_assert(kLutBytes + 12 * kMaxPassPoints <= kMaxDynamicSmem, "eval_exact_kernel's longest pass");
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p)
 {
@@ -878,7 +879,6 @@ constexpr int kSpreadWarps = kSpreadThreads / 32;
 // 338 with 1,024 threads, 394 with 768, compact layout 515 and 427; 150,000 x 200 of 2,048,
 // building, compact: 374 to 464 from one process to the next, and 416).
 __host__ __device__ constexpr int sub_threads(bool dense) { return dense ? 768 : 1024; }
-constexpr size_t kSubSmem = 227 * 1024 - 1024;   // dynamic shared memory beside the static part
 constexpr int kRing = 64;   // deferred lookups per warp (transformed point + scan index)
 constexpr uint32_t kDbgSlow = 0x10000u;   // debug code flag: decided by the exact slow tiers
 
@@ -3051,7 +3051,7 @@ int tiled_warps_per_cta() { return kTiledWarps; }
 
 int tiled_pass_points(const MapView& m, bool dense)
 {
-    const size_t budget = 227 * 1024 - 1024;   // dynamic shared memory left beside the static part
+    const size_t budget = kMaxDynamicSmem;
     size_t fixed = tiled_smem_bytes(m, dense, 0);
     if (fixed >= budget) return 0;
     size_t pts = (budget - fixed) / 12 / 64 * 64;
@@ -3082,7 +3082,7 @@ int launch_eval_pass(const MapView& m, float a_hit, int P, int n0, int n1, int n
     const bool f32 = m.storage != 0;   // value slots (float or half) rather than codes
     if (serial) {
         auto k = f32 ? eval_serial_kernel<true> : eval_serial_kernel<false>;
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (allow_smem(k, kMaxDynamicSmem) != cudaSuccess) return TSDFL_ERR_DEVICE;
         k<<<(P + 255) / 256, 256, smem, s>>>(p);
         g_launches += 1;
     } else if (!f32 && m.tiled && !generic) {
@@ -3123,7 +3123,7 @@ int launch_eval_pass(const MapView& m, float a_hit, int P, int n0, int n1, int n
         int need = (tp.items + kTiledWarps - 1) / kTiledWarps;
         if (need < blocks) blocks = need > 0 ? need : 1;
         auto k = pick_tiled(lay, two, dbg, m.min0 != 0);
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem);
+        if (allow_smem(k, kMaxDynamicSmem) != cudaSuccess) return TSDFL_ERR_DEVICE;
         launch_chained(k, (unsigned)blocks, kTiledThreads, tsmem, s, tp);
         g_launches += 1;
         // the debug kernel scores either kind of cloud; otherwise the one of the
@@ -3138,7 +3138,7 @@ int launch_eval_pass(const MapView& m, float a_hit, int P, int n0, int n1, int n
             sp.items = (unsigned long long)sp.chunks * (unsigned long long)sp.groups;
             const size_t ssmem = spread_smem_bytes(lay == kLayBitmap ? m.occ_bytes : 0u);
             auto ks = pick_spread(lay, two, m.min0 != 0);
-            cudaFuncSetAttribute(ks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssmem);
+            if (allow_smem(ks, kMaxDynamicSmem) != cudaSuccess) return TSDFL_ERR_DEVICE;
             launch_chained(ks, (unsigned)sm_count, kSpreadThreads, ssmem, s, sp);
             g_launches += 1;
         }
@@ -3146,7 +3146,7 @@ int launch_eval_pass(const MapView& m, float a_hit, int P, int n0, int n1, int n
         auto k = dense && !f32 ? eval_exact_kernel<true, 0>
                                : (m.storage == 2 ? eval_exact_kernel<false, 2>
                                                  : (f32 ? eval_exact_kernel<false, 1> : eval_exact_kernel<false, 0>));
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (allow_smem(k, kMaxDynamicSmem) != cudaSuccess) return TSDFL_ERR_DEVICE;
         int blocks = sm_count;
         int need = (P + 31) / 32;
         if (need < blocks) blocks = need > 0 ? need : 1;
@@ -3189,12 +3189,12 @@ int launch_eval_subsample(const MapView& m, float a_hit, int P, int N, int K, un
     size_t smem = (size_t)kLutTableBytes + (dense ? (size_t)m.occ_bytes : 0) + sizeof(float4) * kRing * warps_cta;
     // the scan beside no bitmap, where it fits: 150,000 x 200 of 5,500 points, warehouse,
     // brick table 329 us, 348 from the SoA arrays
-    const bool staged = !dense && smem + sizeof(float4) * (size_t)N <= kSubSmem;
+    const bool staged = !dense && smem + sizeof(float4) * (size_t)N <= kMaxDynamicSmem;
     if (staged) smem += sizeof(float4) * (size_t)N;
     auto k = dense    ? (two ? pick_sub_2<true, true, false>(m.min0 != 0) : pick_sub_2<true, false, false>(m.min0 != 0))
              : staged ? (two ? pick_sub_2<false, true, true>(m.min0 != 0) : pick_sub_2<false, false, true>(m.min0 != 0))
                       : (two ? pick_sub_2<false, true, false>(m.min0 != 0) : pick_sub_2<false, false, false>(m.min0 != 0));
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSubSmem);
+    if (allow_smem(k, kMaxDynamicSmem) != cudaSuccess) return TSDFL_ERR_DEVICE;
     int blocks = sm_count;
     const int need = (P + warps_cta - 1) / warps_cta;
     if (need < blocks) blocks = need > 0 ? need : 1;
@@ -3259,8 +3259,6 @@ uint32_t build_batch_segs(const BatchSegSpec* specs, int nseg, int chunk, int gr
     return total;
 }
 
-size_t batch_smem_bytes() { return 227 * 1024 - 1024; }
-
 // 24 filters (1,000-10,000 particles, 1,000-7,500 points, three maps), scoring and
 // all other kernels of an update: 2.36 ms with one queue of batches of 8 items a
 // warp and barriers around each, 1.94 with batches of 2 or 1, 1.75-1.78 with a
@@ -3269,7 +3267,7 @@ size_t batch_smem_bytes() { return 227 * 1024 - 1024; }
 int launch_eval_batch(void* d_segs, const BatchKinds& kinds, int32_t* status, int sm_count, cudaStream_t s)
 {
     BatchSeg* segs = static_cast<BatchSeg*>(d_segs);
-    const size_t smem = batch_smem_bytes();
+    const size_t smem = kMaxDynamicSmem;
     using BatchKernel = void (*)(BatchSeg*, int, uint32_t, int32_t*);
     static const BatchKernel kKinds[kBatchKinds] = {
         eval_batch_kernel<false, false, false>, eval_batch_kernel<false, true, false>,
@@ -3283,7 +3281,7 @@ int launch_eval_batch(void* d_segs, const BatchKinds& kinds, int32_t* status, in
     for (int kind = 0; kind < kBatchKinds; ++kind) {
         if (kinds.items[kind] == 0) continue;
         auto k = kKinds[kind];
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (allow_smem(k, kMaxDynamicSmem) != cudaSuccess) return TSDFL_ERR_DEVICE;
         // no more CTAs than give every warp an item
         const unsigned blocks =
             std::min((unsigned)sm_count, (kinds.items[kind] + (unsigned)kTiledWarps - 1u) / (unsigned)kTiledWarps);
@@ -3365,13 +3363,17 @@ int launch_resample_impl(const float* particles, const float* w, int stride, siz
     const unsigned blocks = (unsigned)((M + kSumsThreads - 1) / kSumsThreads);
     // small clouds' copies over more SMs
     const int per = blocks >= 128u ? kSumsThreads : (blocks >= 32u ? 256 : 64);
-    launch_chained(resample_scan_kernel, (unsigned)tiles + 1u, kScanThreads, 0, s, w, stride, (int)M, u0, ws);
-    launch_chained(resample_assign_kernel, (unsigned)((M + per - 1) / per), kSumsThreads, 0, s, particles, w, stride,
-                   (int)M, u0, out, idx_out, (long long)cap, count_out, ws, cnt, off, status, per);
-    launch_chained(resample_finish_kernel, blocks, kSumsThreads, 0, s, particles, w, stride, (int)M, out, idx_out,
-                   (long long)cap, count_out, ws, (const uint32_t*)cnt, (const uint32_t*)off, status);
+    // each kernel reads what the one before it wrote: none runs after a failed launch
+    cudaError_t e = launch_chained(resample_scan_kernel, (unsigned)tiles + 1u, kScanThreads, 0, s, w, stride, (int)M, u0, ws);
+    if (e == cudaSuccess)
+        e = launch_chained(resample_assign_kernel, (unsigned)((M + per - 1) / per), kSumsThreads, 0, s, particles, w,
+                           stride, (int)M, u0, out, idx_out, (long long)cap, count_out, ws, cnt, off, status, per);
+    if (e == cudaSuccess)
+        e = launch_chained(resample_finish_kernel, blocks, kSumsThreads, 0, s, particles, w, stride, (int)M, out,
+                           idx_out, (long long)cap, count_out, ws, (const uint32_t*)cnt, (const uint32_t*)off, status);
     g_launches += 3;
-    return check(cudaGetLastError());
+    const cudaError_t last = cudaGetLastError();
+    return check(e == cudaSuccess ? last : e);
 }
 
 int launch_best_particle(const float* particles, size_t M, unsigned long long* key, uint32_t* index_out, int sm_count,

@@ -800,28 +800,36 @@ int launch_resample_residual(const float* particles, const float* w, int stride,
     const long long c = (long long)cap;
     // a draw outside [0, 1) is walked literally
     if (M < kParallelFrom || !(u0 >= 0.0f) || !(u0 < 1.0f)) {
-        launch_chained(residual_chain_kernel, 1, kChainThreads, 0, s, w, stride, m, u0, ws.cnt, ws.off, ws.total,
-                       ws.err);
-        launch_chained(residual_scatter_kernel, (unsigned)((M + 255) / 256), 256, 0, s, particles, m,
-                       (const uint32_t*)ws.cnt, (const uint32_t*)ws.off, (const unsigned long long*)ws.total,
-                       (const int*)ws.err, out, idx_out, c, count_out, status);
+        cudaError_t e = launch_chained(residual_chain_kernel, 1, kChainThreads, 0, s, w, stride, m, u0, ws.cnt, ws.off,
+                                       ws.total, ws.err);
+        if (e == cudaSuccess)
+            e = launch_chained(residual_scatter_kernel, (unsigned)((M + 255) / 256), 256, 0, s, particles, m,
+                               (const uint32_t*)ws.cnt, (const uint32_t*)ws.off,
+                               (const unsigned long long*)ws.total, (const int*)ws.err, out, idx_out, c, count_out,
+                               status);
         g_launches += 2;
-        return check(cudaGetLastError());
+        const cudaError_t last = cudaGetLastError();
+        return check(e == cudaSuccess ? last : e);
     }
     const size_t seg_smem = sizeof(float) * ((size_t)ws.tile + kHead + 4);
     const size_t follow_fixed = sizeof(Seg) * (ws.S + 1) + 4 * (((size_t)ws.S + 1 + 3) / 4 * 4);
     const size_t follow_smem = std::min(kFollowSmem, follow_fixed + 4 * (size_t)ws.S * ws.window);
     ws.staged = (uint32_t)((follow_smem - follow_fixed) / 16 * 4);
-    cudaFuncSetAttribute(residual_follow_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)follow_smem);
-    launch_chained(residual_tiles_kernel, (unsigned)ws.S, kTileThreads, 0, s, w, stride, m, ws);
-    launch_chained(residual_plan_kernel, 1, kPlanThreads, 0, s, m, u0, ws);
-    launch_chained_2d(residual_candidates_kernel, dim3((unsigned)ws.S, (unsigned)(ws.window / kCandThreads)),
-                      kCandThreads, seg_smem, s, w, stride, m, u0, ws);
-    launch_chained(residual_follow_kernel, 1, kChainThreads, follow_smem, s, w, stride, m, u0, ws);
-    launch_chained(residual_emit_kernel, (unsigned)ws.S, kEmitThreads, seg_smem, s, particles, w, stride, m, out,
-                   idx_out, c, count_out, ws, status);
+    if (allow_smem(residual_follow_kernel, kFollowSmem) != cudaSuccess) return TSDFL_ERR_DEVICE;
+    // each kernel reads what the one before it wrote: none runs after a failed launch
+    cudaError_t e = launch_chained(residual_tiles_kernel, (unsigned)ws.S, kTileThreads, 0, s, w, stride, m, ws);
+    if (e == cudaSuccess) e = launch_chained(residual_plan_kernel, 1, kPlanThreads, 0, s, m, u0, ws);
+    if (e == cudaSuccess)
+        e = launch_chained_2d(residual_candidates_kernel, dim3((unsigned)ws.S, (unsigned)(ws.window / kCandThreads)),
+                              kCandThreads, seg_smem, s, w, stride, m, u0, ws);
+    if (e == cudaSuccess)
+        e = launch_chained(residual_follow_kernel, 1, kChainThreads, follow_smem, s, w, stride, m, u0, ws);
+    if (e == cudaSuccess)
+        e = launch_chained(residual_emit_kernel, (unsigned)ws.S, kEmitThreads, seg_smem, s, particles, w, stride, m,
+                           out, idx_out, c, count_out, ws, status);
     g_launches += 5;
-    return check(cudaGetLastError());
+    const cudaError_t last = cudaGetLastError();
+    return check(e == cudaSuccess ? last : e);
 }
 
 }  // namespace tsdfl

@@ -26,6 +26,9 @@ constexpr uint32_t kMissIndex = 0xffffffffu;
 // point); longer scans are evaluated in several passes over point ranges.
 constexpr int kMaxPassPoints = 16384;
 
+// Dynamic shared memory a block may take beside up to 1 KB of static (227 KB in all).
+constexpr size_t kMaxDynamicSmem = 227 * 1024 - 1024;
+
 // Fast-path bound on a map offset (metres): below it float->integer conversions
 // are exact and cannot wrap.
 constexpr float kFastOffsetLimit = 4194304.0f;
