@@ -45,6 +45,14 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes)
                  : "memory");
 }
 
+// After a thread's last plain accesses to shared memory that a bulk copy will write
+// next, before the barrier in front of that copy: bulk copies go another way into
+// shared memory (the async proxy), and a barrier alone does not order the two.
+__device__ __forceinline__ void before_bulk_reuse()
+{
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
 // 1-D bulk copy global -> this CTA's shared memory, completing on bar
 // (cp.async.bulk; src, dst 16-byte aligned, bytes a multiple of 16).
 __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar)
@@ -1643,7 +1651,8 @@ __global__ void __launch_bounds__(kTiledThreads, 1) eval_batch_kernel(BatchSeg* 
                                                                           s_seg.chunk, s_seg.group, chunk, grp,
                                                                           lane);
         }
-        __syncthreads();   // every warp is done with the staged segment
+        before_bulk_reuse();   // the rings' place moves with the segment: the next one's copies may fall on them
+        __syncthreads();       // every warp is done with the staged segment
         if (warp == 0) {
             const int k = batch_most_left(segs, nseg, lane);
             if (lane == 0) s_segi = k;
