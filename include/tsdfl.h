@@ -62,7 +62,9 @@ const char* tsdfl_version(void);
  * process-global, so several maps and contexts can coexist. */
 int tsdfl_ctx_create(int device, tsdfl_ctx** out);
 int tsdfl_ctx_destroy(tsdfl_ctx* ctx);
-/* Use the caller's cudaStream_t (NULL = the context's own stream). */
+/* Use the caller's cudaStream_t (NULL = the context's own stream).  A context's
+ * calls share its workspace: work of two of them must not overlap on the device
+ * (order the streams, and graphs captured from the context, by events). */
 int tsdfl_ctx_set_stream(tsdfl_ctx* ctx, void* cuda_stream);
 void* tsdfl_ctx_stream(tsdfl_ctx* ctx);
 /* Waits for the stream and returns the status raised by device work since the
@@ -499,9 +501,10 @@ uint32_t tsdfl_subsample_index(uint64_t seed, uint64_t particle, uint32_t N, uin
  * call on a device looks the scratch up (cudaGetSymbolAddress), and so does
  * the first call after the device's context changed (cudaDeviceReset): make
  * those calls before any stream capture.  Nothing in the scratch has to start
- * at zero.  Calls
- * whose work overlaps on one device (different streams or host threads with
- * no ordering between them) share the scratch and race: order them. */
+ * at zero (the context's own counters, which every resampling call leaves at
+ * zero, are no part of it).  Calls whose work overlaps on one device (different
+ * streams or host threads with no ordering between them) share the scratch and
+ * race: order them.  Only the results of the calls that overlap are lost. */
 int tsdfl_resample_systematic_static(tsdfl_ctx* ctx, const float* d_particles, size_t M, float u0,
                                      float* d_particles_out, size_t cap, uint32_t* d_count);
 

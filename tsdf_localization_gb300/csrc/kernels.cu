@@ -1977,7 +1977,7 @@ struct ResampleWs {
     double* tile_dsum;      // tiles: double sum of each scan tile's weights (any order)
     int* tile_flag;         // tiles: kTileInexact, kTileWild
     int* err;               // the literal loop would never finish
-    uint32_t* done;         // two block counters, 0 between launches
+    uint32_t* done;         // two block counters, 0 between calls (resample_finish_kernel)
     SumsChunk* chunks;      // ceil(M / kSumsChunk)
 };
 
@@ -2758,6 +2758,9 @@ __global__ void __launch_bounds__(kSumsThreads) resample_finish_kernel(const flo
     chain_enter();
     __shared__ float sw[kSumsChunk];
     __shared__ SumsShared sh;
+    // the counters start the next call at 0, whatever overlapping calls on one context
+    // (whose results race anyway) may have left in them
+    if (blockIdx.x == 0 && threadIdx.x < 2) ws.done[threadIdx.x] = 0u;
     if (*ws.exact_ok) return;
     if (*ws.serial) {
         scatter_block(particles, M, cnt, off, reinterpret_cast<const unsigned long long*>(ws.total), ws.err, out, idx_out,

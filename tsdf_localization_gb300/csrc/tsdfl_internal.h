@@ -331,7 +331,7 @@ int launch_eval_batch(void* d_segs, const BatchKinds& kinds, int32_t* status, in
 // The first of n status words that is not 0 into *sticky, when that is still 0.
 int launch_fold_status(const int32_t* status, int n, int32_t* sticky, cudaStream_t s);
 size_t resample_workspace_bytes(size_t M);
-// done: two counters that are 0 between launches; u0p (optional): the draw read
+// done: two counters that are 0 between calls; u0p (optional): the draw read
 // from device memory when the kernels run.
 int launch_resample_impl(const float* particles, const float* w, int stride, size_t M, float u0, float* out,
                          uint32_t* idx_out, size_t cap, uint32_t* count_out, void* workspace, uint32_t* done,
