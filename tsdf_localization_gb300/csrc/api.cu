@@ -634,6 +634,7 @@ int run_eval(tsdfl_ctx* c, const tsdfl_map* map, const tsdfl_model* mdl, float* 
     const float c_in = mdl->a_range * inv_max_range;
     const float c_out = mdl->a_max;
     const int shift = fixed_shift(map->max_value, (double)N);
+    b.packed = packs(map->max_value, shift);
     const int npad = (int)align_up(N, 4);
     cudaStream_t s = c->stream;
     const bool order = order_particles(P, N);
@@ -689,6 +690,7 @@ int run_eval_sub(tsdfl_ctx* c, const tsdfl_map* map, const tsdfl_model* mdl, flo
     const float c_in = mdl->a_range * inv_max_range;
     const float c_out = mdl->a_max;
     const int shift = fixed_shift(map->max_value, (double)K);
+    b.packed = packs(map->max_value, shift);
     const int npad = (int)align_up(N, 4);
     cudaStream_t s = c->stream;
     const bool order = order_particles(P, K, kOrderFromSub);
@@ -1451,6 +1453,7 @@ void per_configure(tsdfl_batch::Per& q, const tsdfl_filter& F, int sm_count)
     q.b.particles = F.d_particles;
     q.npad = (int)align_up(F.N, 4);
     q.shift = fixed_shift(F.map->max_value, (double)F.N);
+    q.b.packed = packs(F.map->max_value, q.shift);
     const MapView& m = F.map->view;
     q.dense = F.map->occ != nullptr;
     q.tiled = m.storage == 0 && m.tiled != 0;

@@ -691,9 +691,13 @@ __device__ __forceinline__ uint32_t slow_code(const MapView& m, float x, float y
 // Likelihood table entry in shared memory: the fixed-point value of a code,
 // plus 2^kHitShift when the code is a slot's (a hit), so that one 64-bit sum
 // counts both.  The values' part is a signed number below 2^(kHitShift - 1) for
-// up to kPackedLookups lookups (fixed_shift in tsdfl_internal.h sees to it), so
-// unpack() takes the two apart exactly.  Entries 8 bytes apart spread a warp's
-// random reads over 16 bank pairs.
+// up to kPackedLookups lookups, so unpack() takes the two apart exactly.  Entries 8
+// bytes apart spread a warp's random reads over 16 bank pairs.
+// Where the values leave no room for that (packs() in tsdfl_internal.h), the wide
+// form of the kernels (PACKED false) has the values alone in the table and counts
+// the hits by the codes, two instructions a lookup more (building, us, packed / wide:
+// 20,000 x 2,048 162 / 164, 100,000 x 3,000 867 / 888, spread 200,000 x 1,024 1,263 /
+// 1,274).
 struct __align__(8) LutEntry {
     long long v;
 };
@@ -707,6 +711,31 @@ __device__ __forceinline__ void unpack(long long acc, long long& v, uint32_t& hi
 {
     v = (long long)((unsigned long long)acc << (64 - kHitShift)) >> (64 - kHitShift);
     hits = (uint32_t)((unsigned long long)(acc - v) >> kHitShift);
+}
+
+// A lookup's table entry into the lane's sum (packed: with its hit) and, wide, its
+// hit into the lane's count.
+template <bool PACKED>
+__device__ __forceinline__ void take(const LutEntry* lut, uint32_t code, long long& acc, uint32_t& hits)
+{
+    acc += lut[code].v;
+    if (!PACKED) hits += code <= (uint32_t)kCodeInit ? 1u : 0u;
+}
+
+// Moves a packed sum's parts to the lane's 64-bit sum and its hits.
+template <bool PACKED>
+__device__ __forceinline__ void flush(long long& acc, long long& sum, uint32_t& hits)
+{
+    if (PACKED) {
+        long long v;
+        uint32_t h;
+        unpack(acc, v, h);
+        sum += v;
+        hits += h;
+    } else {
+        sum += acc;
+    }
+    acc = 0;
 }
 
 // Settles a lookup the fast path left open where that takes a few compares.
@@ -903,20 +932,42 @@ __device__ __forceinline__ void defer(float4* ring, uint32_t head, uint32_t& tai
 }
 
 // Scores `count` (<= 32) deferred lookups from the ring, one per lane, through
-// the exact second tier / 64-bit emulation; the lane's table entry (packed).  The map view is read from a
-// shared-memory copy so that no kernel parameter's address escapes.
-__device__ __noinline__ long long drain(const MapView* m, const LutEntry* lut, const float4* ring, uint32_t head,
-                                        int count, int lane, uint32_t* dbg_row, const int32_t* perm)
+// the exact second tier / 64-bit emulation: the lane's code, kCodeNone beyond
+// them.  The map view is read from a shared-memory copy so that no kernel
+// parameter's address escapes.
+__device__ __forceinline__ uint32_t drained_code(const MapView* m, const float4* ring, uint32_t head, int count,
+                                                 int lane, uint32_t* dbg_row, const int32_t* perm)
 {
-    long long r = 0;
+    uint32_t code = (uint32_t)kCodeNone;
     if (lane < count) {
         const float4 e = ring[(head + (uint32_t)lane) & (kRing - 1)];
-        const uint32_t code = slow_code(*m, e.x, e.y, e.z);
-        r = lut[code].v;
+        code = slow_code(*m, e.x, e.y, e.z);
         if (dbg_row) dbg_row[perm[__float_as_int(e.w)]] = code | kDbgSlow;
     }
     __syncwarp();
-    return r;
+    return code;
+}
+
+__device__ __noinline__ long long drain_packed(const MapView* m, const LutEntry* lut, const float4* ring,
+                                               uint32_t head, int count, int lane, uint32_t* dbg_row,
+                                               const int32_t* perm)
+{
+    return lut[drained_code(m, ring, head, count, lane, dbg_row, perm)].v;
+}
+
+__device__ __noinline__ uint32_t drain_wide(const MapView* m, const float4* ring, uint32_t head, int count, int lane,
+                                            uint32_t* dbg_row, const int32_t* perm)
+{
+    return drained_code(m, ring, head, count, lane, dbg_row, perm);
+}
+
+template <bool PACKED>
+__device__ __forceinline__ void drain(const MapView* m, const LutEntry* lut, const float4* ring, uint32_t head,
+                                      int count, int lane, uint32_t* dbg_row, const int32_t* perm, long long& acc,
+                                      uint32_t& hits)
+{
+    if (PACKED) acc += drain_packed(m, lut, ring, head, count, lane, dbg_row, perm);
+    else take<false>(lut, drain_wide(m, ring, head, count, lane, dbg_row, perm), acc, hits);
 }
 
 constexpr int kTiledChunk = 1024;     // scan points per work item
@@ -957,7 +1008,8 @@ struct TiledParams {
 // LONG: chunk_pts may exceed 64 kPackedSteps (the batch kernel's, whose steps
 // stay single: in pairs 3.61 against 3.58 ms for 24 filters); otherwise two steps'
 // gathers are in flight at a time.
-template <int LAY, bool TWO, bool DBG, bool MIN0, bool LONG>
+// PACKED: values and hits in one word (LutEntry).
+template <int LAY, bool TWO, bool DBG, bool MIN0, bool LONG, bool PACKED>
 __device__ __forceinline__ void tiled_item(const EvalParams& p, const MapView& m, const MapView* s_map,
                                            const unsigned char* occ, const float4* sxy, const float2* spz,
                                            const LutEntry* lut, float4* ring, int n, int chunk_pts, int group,
@@ -1010,12 +1062,12 @@ __device__ __forceinline__ void tiled_item(const EvalParams& p, const MapView& m
             k1 = s1 ? (uint32_t)kCodeLater : k1;
             defer(ring, head, tail, s0, x0, y0, z0, c0 + 64 * blk + lane, lane);
             if (tail - head >= 32) {
-                acc += drain(s_map, lut, ring, head, 32, lane, dbg_row, perm);
+                drain<PACKED>(s_map, lut, ring, head, 32, lane, dbg_row, perm, acc, hits);
                 head += 32;
             }
             defer(ring, head, tail, s1, x1, y1, z1, c0 + 64 * blk + 32 + lane, lane);
             if (tail - head >= 32) {
-                acc += drain(s_map, lut, ring, head, 32, lane, dbg_row, perm);
+                drain<PACKED>(s_map, lut, ring, head, 32, lane, dbg_row, perm, acc, hits);
                 head += 32;
             }
         };
@@ -1025,7 +1077,8 @@ __device__ __forceinline__ void tiled_item(const EvalParams& p, const MapView& m
                 if (k0 < (uint32_t)kCodeNone) dbg_row[perm[j]] = k0;
                 if (k1 < (uint32_t)kCodeNone) dbg_row[perm[j + 32]] = k1;
             }
-            acc += lut[k0].v + lut[k1].v;
+            take<PACKED>(lut, k0, acc, hits);
+            take<PACKED>(lut, k1, acc, hits);
         };
         // one block (the chunk's partial last one masks its padding points)
         auto step = [&](int blk, bool partial) {
@@ -1059,12 +1112,7 @@ __device__ __forceinline__ void tiled_item(const EvalParams& p, const MapView& m
             for (int blk = 0; blk < nfull;) {
                 const int end = min(blk + kPackedSteps, nfull);
                 for (; blk < end; ++blk) step(blk, false);
-                long long v;
-                uint32_t h;
-                unpack(acc, v, h);
-                sum += v;
-                hits += h;
-                acc = 0;
+                flush<PACKED>(acc, sum, hits);
             }
         } else {
             int blk = 0;
@@ -1073,16 +1121,10 @@ __device__ __forceinline__ void tiled_item(const EvalParams& p, const MapView& m
         }
         if (nfull < nblk) step(nfull, true);
         if (tail != head) {
-            acc += drain(s_map, lut, ring, head, (int)(tail - head), lane, dbg_row, perm);
+            drain<PACKED>(s_map, lut, ring, head, (int)(tail - head), lane, dbg_row, perm, acc, hits);
             head = tail;
         }
-        {
-            long long v;
-            uint32_t h;
-            unpack(acc, v, h);
-            sum += v;
-            hits += h;
-        }
+        flush<PACKED>(acc, sum, hits);
         sum = warp_sum_ll(sum);
         hits = warp_sum_u32(hits);
         if (lane == 0) {
@@ -1094,11 +1136,12 @@ __device__ __forceinline__ void tiled_item(const EvalParams& p, const MapView& m
 
 // Shared memory of the tiled kernels: the likelihood table, the brick bitmap
 // (compact layout), then the staged pass and the deferral rings.
+template <bool PACKED>
 __device__ __forceinline__ void fill_lut(LutEntry* lut, const long long* lut_fx)
 {
     for (int c = threadIdx.x; c < kNumCodes; c += blockDim.x) {
         LutEntry e;
-        e.v = lut_fx[c] + (c <= kCodeInit ? 1ll << kHitShift : 0ll);
+        e.v = lut_fx[c] + (PACKED && c <= kCodeInit ? 1ll << kHitShift : 0ll);
         lut[c] = e;
     }
 }
@@ -1129,7 +1172,7 @@ __device__ __forceinline__ void items_done(uint32_t* work)
 
 // DBG scores any cloud; otherwise a spread cloud is eval_spread_kernel's and this
 // kernel returns at once.
-template <int LAY, bool TWO, bool DBG, bool MIN0>
+template <int LAY, bool TWO, bool DBG, bool MIN0, bool PACKED>
 __global__ void __launch_bounds__(kTiledThreads, 1) eval_tiled_kernel(TiledParams tp)
 {
     chain_enter();
@@ -1147,7 +1190,7 @@ __global__ void __launch_bounds__(kTiledThreads, 1) eval_tiled_kernel(TiledParam
     unsigned char* occ = smem + kLutTableBytes;
     float4* sxy = reinterpret_cast<float4*>(occ + occ_bytes);
     float2* spz = reinterpret_cast<float2*>(sxy + npairs);
-    fill_lut(lut, p.lut_fx);
+    fill_lut<PACKED>(lut, p.lut_fx);
     if (threadIdx.x == 0) mbar_init(&bar, 1);
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1167,8 +1210,8 @@ __global__ void __launch_bounds__(kTiledThreads, 1) eval_tiled_kernel(TiledParam
         const uint32_t item = next_item(tp.work, lane);
         if (item >= (uint32_t)tp.items) break;
         const int chunk = (int)(item / (uint32_t)tp.groups), grp = (int)(item - (uint32_t)chunk * (uint32_t)tp.groups);
-        tiled_item<LAY, TWO, DBG, MIN0, false>(p, m, &s_map, occ, sxy, spz, lut, ring, n, tp.chunk, tp.group,
-                                                     chunk, grp, lane);
+        tiled_item<LAY, TWO, DBG, MIN0, false, PACKED>(p, m, &s_map, occ, sxy, spz, lut, ring, n, tp.chunk, tp.group,
+                                                       chunk, grp, lane);
     }
     items_done(tp.work);
 }
@@ -1188,14 +1231,16 @@ struct SpreadParams {
 
 // Scores `count` (<= 32) deferred lookups, one per lane, and adds each to its
 // own particle (the ring entry's w).
+template <bool PACKED>
 __device__ __noinline__ void drain_to_particles(const MapView* m, const LutEntry* lut, const float4* ring,
                                                 uint32_t head, int count, int lane, long long* sum_fx, uint32_t* hits)
 {
     if (lane < count) {
         const float4 e = ring[(head + (uint32_t)lane) & (kRing - 1)];
-        long long v;
-        uint32_t h;
-        unpack(lut[slow_code(*m, e.x, e.y, e.z)].v, v, h);
+        long long acc = 0, v = 0;
+        uint32_t h = 0;
+        take<PACKED>(lut, slow_code(*m, e.x, e.y, e.z), acc, h);
+        flush<PACKED>(acc, v, h);
         const int pi = __float_as_int(e.w);
         if (v) atomicAdd(reinterpret_cast<unsigned long long*>(sum_fx + pi), (unsigned long long)v);
         if (h) atomicAdd(hits + pi, h);
@@ -1218,7 +1263,7 @@ __device__ __noinline__ void drain_to_particles(const MapView* m, const LutEntry
 // TB/s).  It waits on its gathers now (issue 47 %, L1 tags 48 %): 640 threads of
 // 96 registers 9.1 ms, 768 of 80 9.6; two particles' gathers in flight a warp
 // 10.4, four blocks of points an item 10.6, one 10.2.
-template <int LAY, bool TWO, bool MIN0>
+template <int LAY, bool TWO, bool MIN0, bool PACKED>
 __global__ void __launch_bounds__(kSpreadThreads, 1) eval_spread_kernel(SpreadParams sp)
 {
     chain_enter();
@@ -1236,7 +1281,7 @@ __global__ void __launch_bounds__(kSpreadThreads, 1) eval_spread_kernel(SpreadPa
     float4* ring = reinterpret_cast<float4*>(occ + occ_bytes + kSpreadWarps * (6 * kSpreadGroup) * sizeof(ulonglong2)) +
                    warp * kRing;
     if (threadIdx.x == 0) s_map = m;
-    fill_lut(lut, p.lut_fx);
+    fill_lut<PACKED>(lut, p.lut_fx);
     if (threadIdx.x == 0) mbar_init(&bar, 1);
     __syncthreads();
     bool staged = true;
@@ -1291,8 +1336,8 @@ __global__ void __launch_bounds__(kSpreadThreads, 1) eval_spread_kernel(SpreadPa
             }
         }
         __syncwarp();
-        uint32_t lo = 0, hits = 0;
-        int hi = 0;
+        long long sum = 0;    // of the particle of this lane's place in the group
+        uint32_t hits = 0;
         for (int k = 0; k < kn; ++k) {
             PosePairs R;
 #pragma unroll
@@ -1333,41 +1378,46 @@ __global__ void __launch_bounds__(kSpreadThreads, 1) eval_spread_kernel(SpreadPa
                     c1[b] = s1[b] ? (uint32_t)kCodeLater : c1[b];
                     defer(ring, head, tail, s0[b], x0, y0, z0, who, lane);
                     if (tail - head >= 32) {
-                        drain_to_particles(&s_map, lut, ring, head, 32, lane, p.sum_fx, p.hits);
+                        drain_to_particles<PACKED>(&s_map, lut, ring, head, 32, lane, p.sum_fx, p.hits);
                         head += 32;
                     }
                     defer(ring, head, tail, s1[b], x1, y1, z1, who, lane);
                     if (tail - head >= 32) {
-                        drain_to_particles(&s_map, lut, ring, head, 32, lane, p.sum_fx, p.hits);
+                        drain_to_particles<PACKED>(&s_map, lut, ring, head, 32, lane, p.sum_fx, p.hits);
                         head += 32;
                     }
                 }
             }
-            long long acc = 0;
+            long long acc = 0, v = 0;
+            uint32_t h = 0;
 #pragma unroll
-            for (int b = 0; b < kSpreadBlocks; ++b) acc += lut[c0[b]].v + lut[c1[b]].v;
-            // the warp's sum in parts that cannot overflow: 27 low bits (32 of them
-            // below 2^32), the signed rest (below 2^24 a lane), the hits
-            long long v;
-            uint32_t h;
-            unpack(acc, v, h);
-            const uint32_t l = __reduce_add_sync(0xffffffffu, (uint32_t)v & 0x7ffffffu);
-            const int u = __reduce_add_sync(0xffffffffu, (int)(v >> 27));
+            for (int b = 0; b < kSpreadBlocks; ++b) {
+                take<PACKED>(lut, c0[b], acc, h);
+                take<PACKED>(lut, c1[b], acc, h);
+            }
+            flush<PACKED>(acc, v, h);
             h = __reduce_add_sync(0xffffffffu, h);
+            if (PACKED) {
+                // the warp's sum in parts that cannot overflow: 27 low bits (32 of them
+                // below 2^32) and the signed rest (below 2^25 a lane)
+                const uint32_t l = __reduce_add_sync(0xffffffffu, (uint32_t)v & 0x7ffffffu);
+                const int u = __reduce_add_sync(0xffffffffu, (int)(v >> 27));
+                v = ((long long)u << 27) + (long long)l;
+            } else {
+                v = warp_sum_ll(v);
+            }
             if (lane == k) {
-                lo = l;
-                hi = u;
+                sum = v;
                 hits = h;
             }
         }
         if (lane < kn) {
-            const long long sum = ((long long)hi << 27) + (long long)lo;
             atomicAdd(reinterpret_cast<unsigned long long*>(p.sum_fx + pi), (unsigned long long)sum);
             atomicAdd(p.hits + pi, hits);
         }
         __syncwarp();   // the poses are overwritten by the next item's
     }
-    if (tail != head) drain_to_particles(&s_map, lut, ring, head, (int)(tail - head), lane, p.sum_fx, p.hits);
+    if (tail != head) drain_to_particles<PACKED>(&s_map, lut, ring, head, (int)(tail - head), lane, p.sum_fx, p.hits);
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
@@ -1402,7 +1452,7 @@ struct SubParams {
     int group, items;    // particles an item, items
 };
 
-template <bool DENSE, bool TWO, bool MIN0, bool STAGED>
+template <bool DENSE, bool TWO, bool MIN0, bool STAGED, bool PACKED>
 __global__ void __launch_bounds__(sub_threads(DENSE), 1) eval_subsample_kernel(SubParams sp)
 {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -1416,7 +1466,7 @@ __global__ void __launch_bounds__(sub_threads(DENSE), 1) eval_subsample_kernel(S
     float4* rings = reinterpret_cast<float4*>(occ + occ_bytes);
     float4* pts = rings + kRing * (sub_threads(DENSE) / 32);
     if (threadIdx.x == 0) s_map = m;
-    fill_lut(lut, p.lut_fx);
+    fill_lut<PACKED>(lut, p.lut_fx);
     if (STAGED)
         for (int j = threadIdx.x; j < p.n_total; j += sub_threads(DENSE))
             pts[j] = make_float4(p.xs[j], p.ys[j], p.zs[j], p.cs[j]);
@@ -1504,7 +1554,7 @@ __global__ void __launch_bounds__(sub_threads(DENSE), 1) eval_subsample_kernel(S
                 k0 = s0 ? (uint32_t)kCodeLater : k0;
                 defer(ring, head, tail, s0, tx, ty, tz, (int)ja, lane);
                 if (tail - head >= 32) {
-                    acc += drain(&s_map, lut, ring, head, 32, lane, nullptr, nullptr);
+                    drain<PACKED>(&s_map, lut, ring, head, 32, lane, nullptr, nullptr, acc, hits);
                     head += 32;
                 }
                 upk(TX, u, tx); upk(TY, u, ty); upk(TZ, u, tz);
@@ -1512,30 +1562,22 @@ __global__ void __launch_bounds__(sub_threads(DENSE), 1) eval_subsample_kernel(S
                 k1 = s1 ? (uint32_t)kCodeLater : k1;
                 defer(ring, head, tail, s1, tx, ty, tz, (int)jb, lane);
                 if (tail - head >= 32) {
-                    acc += drain(&s_map, lut, ring, head, 32, lane, nullptr, nullptr);
+                    drain<PACKED>(&s_map, lut, ring, head, 32, lane, nullptr, nullptr, acc, hits);
                     head += 32;
                 }
             }
-            const LutEntry e0 = lut[k0], e1 = lut[k1];
-            acc += e0.v + e1.v;
+            take<PACKED>(lut, k0, acc, hits);
+            take<PACKED>(lut, k1, acc, hits);
             if (++packed == kPackedSteps) {
-                long long v;
-                uint32_t h;
-                unpack(acc, v, h);
-                sum += v;
-                hits += h;
-                acc = 0;
+                flush<PACKED>(acc, sum, hits);
                 packed = 0;
             }
         }
-        if (tail != head) acc += drain(&s_map, lut, ring, head, (int)(tail - head), lane, nullptr, nullptr);
-        {
-            long long v;
-            uint32_t h;
-            unpack(acc, v, h);
-            sum = warp_sum_ll(sum + v);
-            hits = warp_sum_u32(hits + h);
-        }
+        if (tail != head)
+            drain<PACKED>(&s_map, lut, ring, head, (int)(tail - head), lane, nullptr, nullptr, acc, hits);
+        flush<PACKED>(acc, sum, hits);
+        sum = warp_sum_ll(sum);
+        hits = warp_sum_u32(hits);
         nin = warp_sum_u32(nin);
         if (lane == 0) {
             p.sum_fx[pi] = sum;
@@ -1600,7 +1642,7 @@ __device__ __forceinline__ int batch_most_left(const BatchSeg* segs, int nseg, i
 // when no segment has an item left, so none is missed.  Per-item scoring is
 // eval_tiled_kernel's, so every filter's sums equal its single-filter sums bit for
 // bit.
-template <bool DENSE, bool TWO, bool MIN0>
+template <bool DENSE, bool TWO, bool MIN0, bool PACKED>
 __global__ void __launch_bounds__(kTiledThreads, 1) eval_batch_kernel(BatchSeg* segs, int nseg, uint32_t total_items,
                                                                       int32_t* status)
 {
@@ -1631,7 +1673,7 @@ __global__ void __launch_bounds__(kTiledThreads, 1) eval_batch_kernel(BatchSeg* 
         float4* sxy = reinterpret_cast<float4*>(occ + occ_bytes);
         float2* spz = reinterpret_cast<float2*>(sxy + npairs);
         float4* ring = reinterpret_cast<float4*>(spz + npairs) + warp * kRing;
-        fill_lut(lut, p.lut_fx);
+        fill_lut<PACKED>(lut, p.lut_fx);
         if (threadIdx.x == 0) {
             mbar_expect_tx(&bar, (uint32_t)npairs * 24u + occ_bytes);
             bulk_g2s(sxy, p.pxy + p.n0 / 2, (uint32_t)npairs * 16u, &bar);
@@ -1647,9 +1689,8 @@ __global__ void __launch_bounds__(kTiledThreads, 1) eval_batch_kernel(BatchSeg* 
             const uint32_t item = next_item(&segs[segi].next, lane);
             if (item >= (uint32_t)s_seg.items) break;
             const int chunk = (int)item / s_seg.groups, grp = (int)item - chunk * s_seg.groups;
-            tiled_item<DENSE ? kLayBitmap : kLayTable, TWO, false, MIN0, true>(p, p.m, &p.m, occ, sxy, spz, lut, ring, n,
-                                                                          s_seg.chunk, s_seg.group, chunk, grp,
-                                                                          lane);
+            tiled_item<DENSE ? kLayBitmap : kLayTable, TWO, false, MIN0, true, PACKED>(
+                p, p.m, &p.m, occ, sxy, spz, lut, ring, n, s_seg.chunk, s_seg.group, chunk, grp, lane);
         }
         before_bulk_reuse();   // the rings' place moves with the segment: the next one's copies may fall on them
         __syncthreads();       // every warp is done with the staged segment
@@ -3011,45 +3052,54 @@ size_t eval_smem_bytes(bool serial, int n)
 
 using TiledKernel = void (*)(TiledParams);
 
+// The wide and the debug kernels come without the shortcut for a min corner at the
+// origin, and the debug ones wide only: sums and hits are the same.
 template <int LAY, bool TWO>
-TiledKernel pick_tiled_2(bool dbg, bool min0)
+TiledKernel pick_tiled_2(bool dbg, bool min0, bool packed)
 {
-    if (dbg) return min0 ? eval_tiled_kernel<LAY, TWO, true, true> : eval_tiled_kernel<LAY, TWO, true, false>;
-    return min0 ? eval_tiled_kernel<LAY, TWO, false, true> : eval_tiled_kernel<LAY, TWO, false, false>;
+    if (dbg) return eval_tiled_kernel<LAY, TWO, true, false, false>;
+    if (!packed) return eval_tiled_kernel<LAY, TWO, false, false, false>;
+    return min0 ? eval_tiled_kernel<LAY, TWO, false, true, true> : eval_tiled_kernel<LAY, TWO, false, false, true>;
 }
 
 template <int LAY>
-TiledKernel pick_tiled_1(bool two, bool dbg, bool min0)
+TiledKernel pick_tiled_1(bool two, bool dbg, bool min0, bool packed)
 {
-    return two ? pick_tiled_2<LAY, true>(dbg, min0) : pick_tiled_2<LAY, false>(dbg, min0);
+    return two ? pick_tiled_2<LAY, true>(dbg, min0, packed) : pick_tiled_2<LAY, false>(dbg, min0, packed);
 }
 
-TiledKernel pick_tiled(int lay, bool two, bool dbg, bool min0)
+TiledKernel pick_tiled(int lay, bool two, bool dbg, bool min0, bool packed)
 {
     switch (lay) {
-    case kLayBitmap: return pick_tiled_1<kLayBitmap>(two, dbg, min0);
-    case kLayHash: return pick_tiled_1<kLayHash>(two, dbg, min0);
-    case kLayGrid: return pick_tiled_1<kLayGrid>(two, dbg, min0);
-    default: return pick_tiled_1<kLayTable>(two, dbg, min0);
+    case kLayBitmap: return pick_tiled_1<kLayBitmap>(two, dbg, min0, packed);
+    case kLayHash: return pick_tiled_1<kLayHash>(two, dbg, min0, packed);
+    case kLayGrid: return pick_tiled_1<kLayGrid>(two, dbg, min0, packed);
+    default: return pick_tiled_1<kLayTable>(two, dbg, min0, packed);
     }
 }
 
 using SpreadKernel = void (*)(SpreadParams);
 
-template <int LAY>
-SpreadKernel pick_spread_1(bool two, bool min0)
+template <int LAY, bool TWO>
+SpreadKernel pick_spread_2(bool min0, bool packed)
 {
-    if (two) return min0 ? eval_spread_kernel<LAY, true, true> : eval_spread_kernel<LAY, true, false>;
-    return min0 ? eval_spread_kernel<LAY, false, true> : eval_spread_kernel<LAY, false, false>;
+    if (!packed) return eval_spread_kernel<LAY, TWO, false, false>;
+    return min0 ? eval_spread_kernel<LAY, TWO, true, true> : eval_spread_kernel<LAY, TWO, false, true>;
 }
 
-SpreadKernel pick_spread(int lay, bool two, bool min0)
+template <int LAY>
+SpreadKernel pick_spread_1(bool two, bool min0, bool packed)
+{
+    return two ? pick_spread_2<LAY, true>(min0, packed) : pick_spread_2<LAY, false>(min0, packed);
+}
+
+SpreadKernel pick_spread(int lay, bool two, bool min0, bool packed)
 {
     switch (lay) {
-    case kLayBitmap: return pick_spread_1<kLayBitmap>(two, min0);
-    case kLayHash: return pick_spread_1<kLayHash>(two, min0);
-    case kLayGrid: return pick_spread_1<kLayGrid>(two, min0);
-    default: return pick_spread_1<kLayTable>(two, min0);
+    case kLayBitmap: return pick_spread_1<kLayBitmap>(two, min0, packed);
+    case kLayHash: return pick_spread_1<kLayHash>(two, min0, packed);
+    case kLayGrid: return pick_spread_1<kLayGrid>(two, min0, packed);
+    default: return pick_spread_1<kLayTable>(two, min0, packed);
     }
 }
 
@@ -3134,7 +3184,7 @@ int launch_eval_pass(const MapView& m, float a_hit, int P, int n0, int n1, int n
         int blocks = sm_count;
         int need = (tp.items + kTiledWarps - 1) / kTiledWarps;
         if (need < blocks) blocks = need > 0 ? need : 1;
-        auto k = pick_tiled(lay, two, dbg, m.min0 != 0);
+        auto k = pick_tiled(lay, two, dbg, m.min0 != 0, b.packed != 0);
         if (allow_smem(k, kMaxDynamicSmem) != cudaSuccess) return TSDFL_ERR_DEVICE;
         launch_chained(k, (unsigned)blocks, kTiledThreads, tsmem, s, tp);
         g_launches += 1;
@@ -3149,7 +3199,7 @@ int launch_eval_pass(const MapView& m, float a_hit, int P, int n0, int n1, int n
             sp.groups = (P + kSpreadGroup - 1) / kSpreadGroup;
             sp.items = (unsigned long long)sp.chunks * (unsigned long long)sp.groups;
             const size_t ssmem = spread_smem_bytes(lay == kLayBitmap ? m.occ_bytes : 0u);
-            auto ks = pick_spread(lay, two, m.min0 != 0);
+            auto ks = pick_spread(lay, two, m.min0 != 0, b.packed != 0);
             if (allow_smem(ks, kMaxDynamicSmem) != cudaSuccess) return TSDFL_ERR_DEVICE;
             launch_chained(ks, (unsigned)sm_count, kSpreadThreads, ssmem, s, sp);
             g_launches += 1;
@@ -3168,10 +3218,20 @@ int launch_eval_pass(const MapView& m, float a_hit, int P, int n0, int n1, int n
     return check(cudaGetLastError());
 }
 
+using SubKernel = void (*)(SubParams);
+
 template <bool DENSE, bool TWO, bool STAGED>
-void (*pick_sub_2(bool min0))(SubParams)
+SubKernel pick_sub_2(bool min0, bool packed)
 {
-    return min0 ? eval_subsample_kernel<DENSE, TWO, true, STAGED> : eval_subsample_kernel<DENSE, TWO, false, STAGED>;
+    if (!packed) return eval_subsample_kernel<DENSE, TWO, false, STAGED, false>;
+    return min0 ? eval_subsample_kernel<DENSE, TWO, true, STAGED, true>
+                : eval_subsample_kernel<DENSE, TWO, false, STAGED, true>;
+}
+
+template <bool DENSE, bool STAGED>
+SubKernel pick_sub(bool two, bool min0, bool packed)
+{
+    return two ? pick_sub_2<DENSE, true, STAGED>(min0, packed) : pick_sub_2<DENSE, false, STAGED>(min0, packed);
 }
 
 int launch_eval_subsample(const MapView& m, float a_hit, int P, int N, int K, unsigned long long seed, float c_in,
@@ -3203,9 +3263,10 @@ int launch_eval_subsample(const MapView& m, float a_hit, int P, int N, int K, un
     // brick table 329 us, 348 from the SoA arrays
     const bool staged = !dense && smem + sizeof(float4) * (size_t)N <= kMaxDynamicSmem;
     if (staged) smem += sizeof(float4) * (size_t)N;
-    auto k = dense    ? (two ? pick_sub_2<true, true, false>(m.min0 != 0) : pick_sub_2<true, false, false>(m.min0 != 0))
-             : staged ? (two ? pick_sub_2<false, true, true>(m.min0 != 0) : pick_sub_2<false, false, true>(m.min0 != 0))
-                      : (two ? pick_sub_2<false, true, false>(m.min0 != 0) : pick_sub_2<false, false, false>(m.min0 != 0));
+    const bool min0 = m.min0 != 0, packed = b.packed != 0;
+    const SubKernel k = dense    ? pick_sub<true, false>(two, min0, packed)
+                        : staged ? pick_sub<false, true>(two, min0, packed)
+                                 : pick_sub<false, false>(two, min0, packed);
     if (allow_smem(k, kMaxDynamicSmem) != cudaSuccess) return TSDFL_ERR_DEVICE;
     int blocks = sm_count;
     const int need = (P + warps_cta - 1) / warps_cta;
@@ -3233,13 +3294,13 @@ uint32_t build_batch_segs(const BatchSegSpec* specs, int nseg, int chunk, int gr
     });
     uint32_t total = 0;
     int o = 0;
-    for (int kind = 0; kind < kBatchKinds; ++kind) {   // bit 2: min at the origin, bit 1: compact, bit 0: two-term
+    for (int kind = 0; kind < kBatchKinds; ++kind) {
         kinds->first[kind] = o;
         kinds->count[kind] = 0;
         uint32_t batches = 0, items = 0;
         for (int oi = 0; oi < nseg; ++oi) {
             const BatchSegSpec& sp = specs[order[oi]];
-            const int k = (sp.m.min0 ? 4 : 0) + (sp.dense ? 2 : 0) + (sp.m.sub_fast == 1 ? 1 : 0);
+            const int k = (!sp.b.packed ? 8 : (sp.m.min0 ? 4 : 0)) + (sp.dense ? 2 : 0) + (sp.m.sub_fast == 1 ? 1 : 0);
             if (k != kind) continue;
             const EvalBuffers& b = sp.b;
             BatchSeg g{};
@@ -3282,10 +3343,12 @@ int launch_eval_batch(void* d_segs, const BatchKinds& kinds, int32_t* status, in
     const size_t smem = kMaxDynamicSmem;
     using BatchKernel = void (*)(BatchSeg*, int, uint32_t, int32_t*);
     static const BatchKernel kKinds[kBatchKinds] = {
-        eval_batch_kernel<false, false, false>, eval_batch_kernel<false, true, false>,
-        eval_batch_kernel<true, false, false>,  eval_batch_kernel<true, true, false>,
-        eval_batch_kernel<false, false, true>,  eval_batch_kernel<false, true, true>,
-        eval_batch_kernel<true, false, true>,   eval_batch_kernel<true, true, true>};
+        eval_batch_kernel<false, false, false, true>,  eval_batch_kernel<false, true, false, true>,
+        eval_batch_kernel<true, false, false, true>,   eval_batch_kernel<true, true, false, true>,
+        eval_batch_kernel<false, false, true, true>,   eval_batch_kernel<false, true, true, true>,
+        eval_batch_kernel<true, false, true, true>,    eval_batch_kernel<true, true, true, true>,
+        eval_batch_kernel<false, false, false, false>, eval_batch_kernel<false, true, false, false>,
+        eval_batch_kernel<true, false, false, false>,  eval_batch_kernel<true, true, false, false>};
     int nseg = 0;
     for (int kind = 0; kind < kBatchKinds; ++kind) nseg += kinds.count[kind];
     if (nseg == 0) return TSDFL_OK;

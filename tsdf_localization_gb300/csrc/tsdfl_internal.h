@@ -192,20 +192,25 @@ static __device__ __forceinline__ void transform_point(const float* t, float x, 
 
 #endif  // __CUDACC__
 
+// Fixed-point scale 2^shift of the likelihood sums of n lookups of values up to
+// max_value in magnitude: at most 2^40, the sum of n + 1 below 2^62.
+inline int fixed_shift(double max_value, double n)
+{
+    const double top = std::fmax(max_value, 1e-30);
+    return std::min(40, 62 - (int)std::ceil(std::log2(top * (n + 1.0))));
+}
+
 // Lookups a lane of the tiled kernels sums in one 64-bit word that holds the
 // values in its lower 57 bits (signed) and the hits above them.
 constexpr int kPackedLookups = 72;
 
-// Fixed-point scale 2^shift of the likelihood sums of n lookups of values up
-// to max_value in magnitude: at most 2^40, the sum of n + 1 below 2^62, and the
-// sum of kPackedLookups below 2^56 (without effect for a sigma of 0.042 m and
-// more; below, shorter scans get the scale a scan of 4,608 points has anyway).
-inline int fixed_shift(double max_value, double n)
+// Whether so many lookups sum below 2^56 at that scale.  They do for a sigma of
+// 0.042 m and more, and below it for scans of some 4,000 points and more, whose own
+// sum needs the room; the tiled kernels' wide form, which counts the hits beside the
+// sum, scores the others.
+inline bool packs(double max_value, int shift)
 {
-    const double top = std::fmax(max_value, 1e-30);
-    const int sum = 62 - (int)std::ceil(std::log2(top * (n + 1.0)));
-    const int packed = 56 - (int)std::ceil(std::log2(top * kPackedLookups));
-    return std::min(40, std::min(sum, packed));
+    return shift + (int)std::ceil(std::log2(std::fmax(max_value, 1e-30) * kPackedLookups)) <= 56;
 }
 
 // EvalBuffers::work: [0, 1] the tiled kernel's item counter and CTAs done,
@@ -257,6 +262,7 @@ struct EvalBuffers {
     float* lut_f;            // kNumCodes float likelihoods
     int32_t* counts;         // [0] = points in range
     uint32_t* work;          // kWorkWords: item counters of the tiled kernels, 0 between launches
+    int packed;              // packs(): the tiled kernels sum values and hits in one word
     double* partials;        // reduction partials
     double* sums;            // [0] weight sum, [1..9] pose sums
     float* weight_sum_f;     // [1]
@@ -313,10 +319,10 @@ struct BatchSegSpec {
     bool dense;
     EvalBuffers b;
 };
-// The segments of each map-layout kind (bit 2: min corner at the origin, bit 1:
-// compact layout, bit 0: two-term sub-voxel multiplier) form one queue and one
-// persistent launch.
-constexpr int kBatchKinds = 8;
+// The segments of each kind (bit 3: wide sums, whatever the min corner; bit 2: min
+// corner at the origin, bit 1: compact layout, bit 0: two-term sub-voxel multiplier)
+// form one queue and one persistent launch.
+constexpr int kBatchKinds = 12;
 struct BatchKinds {
     int first[kBatchKinds], count[kBatchKinds];
     uint32_t items[kBatchKinds];
