@@ -42,6 +42,7 @@ struct MotionParams {
     uint32_t P;
     double mean[6], stddev[6];
     Pair mean2[6], stddev2[6];
+    float low[6];            // normal_draw's
     int pairs;               // mean and stddev lie where pairs hold their digits
     unsigned long long key0, key1, step;
     const double* draws;     // P x 6 given draws, or null: generate
@@ -259,9 +260,9 @@ __global__ void __launch_bounds__(kMotionBlock) motion_kernel(const __grid_const
             const bool ok = normal_pairs(w[k], w[k + 1], z[0], z[1]);
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-                const Pair n = mul(z[j], mp.stddev2[k + j]);
-                d[k + j].v = add(n, mp.mean2[k + j]);
-                d[k + j].bound = ok ? (fabsf(n.h) + fabsf(mp.mean2[k + j].h)) * kPairRel : __int_as_float(0x7fffffff);
+                float bound;
+                d[k + j].v = normal_draw(z[j], mp.stddev2[k + j], mp.mean2[k + j], mp.low[k + j], bound);
+                d[k + j].bound = ok ? bound : __int_as_float(0x7fffffff);
             }
         }
     } else {
@@ -343,6 +344,7 @@ int launch_motion(float* particles, size_t P, const double mean[6], const double
         if (mp.pairs) {
             mp.mean2[k] = from_double(mp.mean[k]);
             mp.stddev2[k] = from_double(mp.stddev[k]);
+            mp.low[k] = mp.stddev[k] != 0.0 ? kDrawLow : 0.0f;
         }
     }
     mp.key0 = seed;

@@ -258,4 +258,16 @@ PAIR_FN bool normal_pairs(uint64_t a, uint64_t b, Pair& z0, Pair& z1)
     return true;
 }
 
+// The draw z stddev + mean of a normal z (normal_pairs), and the bound it is known to.
+// `low` is kDrawLow for a stddev above 0, else 0: where z stddev is tiny the products'
+// low parts leave the normal range, and the relative part of the bound with them.  The
+// parts lost there are a few units of 2^-149; from 2^-75 up kDrawLow adds nothing.
+constexpr float kDrawLow = 0x1p-120f;
+PAIR_FN Pair normal_draw(Pair z, Pair stddev, Pair mean, float low, float& bound)
+{
+    const Pair n = mul(z, stddev);
+    bound = fmaf(fabsf(n.h) + fabsf(mean.h), kPairRel, low);
+    return add(n, mean);
+}
+
 }  // namespace tsdfl
