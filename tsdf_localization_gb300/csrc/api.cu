@@ -417,6 +417,9 @@ void fill_view(tsdfl_map* m)
     // negative sub-voxel index (an empty range when not even layer 0 passes)
     v.zhi = v.mmax_z < 0 ? 0.0f : (float)std::min<int64_t>((int64_t)v.mmax_z + 1, 4194304);
     v.zlo = v.mmax_z < 0 ? 0.0f : -1.0f;
+    // the points below a grid layout where coordinates past the last brick of the
+    // lowest layer alias into the next one (whose bricks have no skirt) are the slow tiers'
+    if (m->grid && brick_reach(c, 1) > c.up_dim_2) v.zlo = std::fmax(v.zlo, std::nextafter(0.0f, -1.0f));
     float far[4];
     miss_bounds(c, v.mmax_x, v.mmax_y, far);
     v.far_limit = far[0];
@@ -449,10 +452,8 @@ int build_grid(tsdfl_map* m, cudaStream_t s)
 {
     const tsdfl_map_coef& c = m->coef;
     const uint64_t S3 = c.sub_dim * c.sub_dim_2;
-    // where coordinates past the last brick of a row alias into the next one, a
-    // lookup below the floor can reach a brick that has no skirt
     if (max_sub_index(c.resolution) >= c.sub_dim || !m->codes || m->codes_pre != S3 || c.grid_occ_size == 0 ||
-        c.grid_occ_size >= (1ull << 23) || brick_reach(c) > c.grid_occ_size)
+        c.grid_occ_size >= (1ull << 23))
         return TSDFL_OK;
     const uint64_t n = (c.grid_occ_size + c.up_dim_2) * S3;
     if (n >= (1ull << 31)) return TSDFL_OK;

@@ -117,13 +117,14 @@ int32_t coarse_mmax(uint64_t dim, float res)
     return 4194304;
 }
 
-uint64_t brick_reach(const tsdfl_map_coef& c)
+uint64_t brick_reach(const tsdfl_map_coef& c, uint64_t layers)
 {
     auto last = [&](uint64_t dim) {
         const int32_t m = coarse_mmax(dim, c.resolution);
         return m < 0 ? 0ull : (uint64_t)std::min<int32_t>(m, 4194303);
     };
-    return last(c.dim_x) + last(c.dim_y) * c.up_dim_x + last(c.dim_z) * c.up_dim_2 + 1;
+    const uint64_t z = std::min<uint64_t>(last(c.dim_z), layers ? layers - 1 : 0);
+    return last(c.dim_x) + last(c.dim_y) * c.up_dim_x + z * c.up_dim_2 + 1;
 }
 
 void miss_bounds(const tsdfl_map_coef& c, int32_t mmax_x, int32_t mmax_y, float far[4])

@@ -20,8 +20,8 @@ uint64_t host_slot_index(const tsdfl_map_coef& c, const int32_t* grid_occ, float
 int32_t coarse_mmax(uint64_t dim, float res);
 // One past the largest brick index trunc(ox) + trunc(oy) up_dim_x + trunc(oz)
 // up_dim_2 of offsets that pass the coarse bound check (coarse_mmax, capped at
-// 2^22 m) on every axis.
-uint64_t brick_reach(const tsdfl_map_coef& c);
+// 2^22 m) on every axis, with trunc(oz) below `layers`.
+uint64_t brick_reach(const tsdfl_map_coef& c, uint64_t layers = UINT64_MAX);
 // Bounds below which an offset settles a miss whatever the other axes hold, as
 // long as every offset lies below far[0] in magnitude: far[1] on x (an odd
 // multiple of 2^63 in the slot index, where sub_dim is even), far[2] on y with
