@@ -1,6 +1,7 @@
 """Maps whose last brick coordinate that passes the coarse check lies past the brick
 table (sizes of whole metres at a resolution that does not divide them): they get the
-grid layout when they ask for it and score as the generic kernel does, below the floor, above the top and past the sides."""
+layout that was asked for -- the grid, and the bitmap up to its largest size -- and
+score as the generic kernel does, below the floor, above the top and past the sides."""
 import numpy as np
 import pytest
 
@@ -9,7 +10,7 @@ from tsdf_localization_gb300 import Context, DeviceMap, TSDFEvaluator, synth
 from test_gpu_scoring_kernels import cloud, random_map, scan
 
 pytestmark = pytest.mark.gpu
-GRID = 3
+GRID, BITMAP, HASH = 3, 1, 2
 
 
 @pytest.fixture(scope="module")
@@ -52,4 +53,19 @@ def test_grid_layout(ctx, size, res):
         assert aliases(coef, axis) == (s == int(s))
     dmap = DeviceMap(ctx, coef, occ, codes=codes, grid=True)
     assert dmap.info()["dense"] == GRID
+    check(ctx, dmap, size, rng, CLOUDS)
+
+
+@pytest.mark.parametrize("size,layout,table", [((100.0, 100.0, 52.0), BITMAP, 1 << 17), ((70.0, 71.0, 52.0), BITMAP, 1 << 16),
+                                               ((100.0, 100.0, 53.0), HASH, 0), ((30.0, 31.0, 9.0), BITMAP, 1 << 12)])
+def test_bitmap_up_to_its_largest_size(ctx, size, layout, table):
+    """520,000 bricks of at most 524,288; 258,440 of the 262,144 of half the table."""
+    rng = np.random.default_rng(2)
+    coef, occ, codes = random_map(size, 0.3, (0, 0, 0), 2)
+    assert aliases(coef, "z")
+    plain = DeviceMap(ctx, coef, occ, codes=codes)
+    dmap = DeviceMap(ctx, coef, occ, codes=codes, dense=True)
+    assert dmap.info()["dense"] == layout
+    if table:
+        assert dmap.info()["device_bytes"] - plain.info()["device_bytes"] == table
     check(ctx, dmap, size, rng, CLOUDS)

@@ -100,6 +100,7 @@ struct tsdfl_map {
     uint2* hash = nullptr;        // sparse brick hash (TSDFL_MAP_HASH, or DENSE with a bitmap too large)
     uint16_t* grid = nullptr;     // grid layout (TSDFL_MAP_GRID): every brick of the bounding box
     uint64_t grid_codes = 0;      // codes in grid before the sentinels
+    uint64_t fast_layers = UINT64_MAX;   // brick layers whose indices the bitmap covers
     uint32_t hash_slots = 0, hash_probes = 0;
     float* values = nullptr;      // kNumCodes likelihood values (device)
     float max_value = 0;
@@ -417,8 +418,10 @@ void fill_view(tsdfl_map* m)
     // negative sub-voxel index (an empty range when not even layer 0 passes)
     v.zhi = v.mmax_z < 0 ? 0.0f : (float)std::min<int64_t>((int64_t)v.mmax_z + 1, 4194304);
     v.zlo = v.mmax_z < 0 ? 0.0f : -1.0f;
-    // the points below a grid layout where coordinates past the last brick of the
-    // lowest layer alias into the next one (whose bricks have no skirt) are the slow tiers'
+    // the layers past the bitmap's, and the points below a grid layout where
+    // coordinates past the last brick of the lowest layer alias into the next one
+    // (whose bricks have no skirt), are the slow tiers'
+    if (m->occ && m->fast_layers < 4194304) v.zhi = std::fmin(v.zhi, (float)m->fast_layers);
     if (m->grid && brick_reach(c, 1) > c.up_dim_2) v.zlo = std::fmax(v.zlo, std::nextafter(0.0f, -1.0f));
     float far[4];
     miss_bounds(c, v.mmax_x, v.mmax_y, far);
@@ -477,10 +480,18 @@ int build_compact(tsdfl_map* m, const int32_t* go)
     const uint64_t gos = c.grid_occ_size;
     if (max_sub_index(c.resolution) >= c.sub_dim || !m->codes || m->codes_pre != c.sub_dim * c.sub_dim_2)
         return TSDFL_OK;   // brick table only
-    // zero words for every brick index a lookup inside the fast domain can form
-    const uint64_t words = (std::max(gos, brick_reach(c)) + 31) / 32;
-    uint64_t bytes = 16;
-    while (bytes < 8 * words && bytes <= (1u << 17)) bytes *= 2;
+    // zero words for every brick index a lookup inside the fast domain can form; a
+    // table that only the layers past the last brick make larger goes without them
+    uint64_t words = 0, bytes = 0;
+    auto size_to = [&](uint64_t reach) {
+        words = (std::max(gos, reach) + 31) / 32;
+        for (bytes = 16; bytes < 8 * words && bytes <= (1u << 17);) bytes *= 2;
+    };
+    size_to(brick_reach(c));
+    const uint64_t full = bytes;
+    size_to(brick_reach(c, c.up_dim_z));
+    if (bytes < full) m->fast_layers = c.up_dim_z;
+    else size_to(brick_reach(c));
     if (bytes > (1u << 17)) return TSDFL_OK;
     std::vector<uint32_t> occ(bytes / 4, 0u);
     for (uint64_t up = 0; up < gos; ++up)
