@@ -71,7 +71,8 @@ void* tsdfl_ctx_stream(tsdfl_ctx* ctx);
  * last sync (e.g. TSDFL_ERR_DEGENERATE from tsdfl_evaluate_device). */
 int tsdfl_ctx_sync(tsdfl_ctx* ctx);
 /* Pre-sizes the workspace for P particles and N points so that later calls
- * with at most as many allocate nothing. */
+ * with at most as many allocate nothing (the residual systematic resampler's
+ * tables among it: 24 MB at a million particles, 134 MB at 2^24). */
 int tsdfl_ctx_reserve(tsdfl_ctx* ctx, size_t P, size_t N);
 
 /* Device timing of the scoring kernels of the next evaluations (CUDA events
@@ -235,7 +236,8 @@ int tsdfl_resample_systematic_device(tsdfl_ctx* ctx, const float* d_particles, s
  * particle m is emitted (size_t)(temp + 1.0) times, temp = (float)M * w_m - u,
  * u then becomes (float)count - temp.  Bit-exact with the reference for the
  * same weights and u0 (large clouds walk the float chain's likely starts in
- * parallel, small ones one thread walks it).  Negative or non-finite weights, or
+ * parallel; one thread walks it for small ones, and where the tables of the
+ * parallel form cannot be allocated: first used while the stream is captured).  Negative or non-finite weights, or
  * a particle count of 2^24, give TSDFL_ERR_UNSUPPORTED. */
 int tsdfl_resample_residual_systematic(tsdfl_ctx* ctx, const float* weights, size_t M, float u0, uint32_t* idx_out,
                                        size_t cap, size_t* count_out);

@@ -70,6 +70,8 @@ struct tsdfl_ctx {
     size_t ws_bytes = 0;
     void* rs_ws = nullptr;       // resampling workspace
     size_t rs_bytes = 0;
+    void* rt_ws = nullptr;       // residual systematic resampling: the candidates' tables
+    size_t rt_bytes = 0;
     void* scan_ws = nullptr;     // scan reduction workspace
     size_t scan_bytes = 0;
     void* aux_ws = nullptr;      // workspace of the other resamplers
@@ -211,9 +213,11 @@ int ensure_workspace(tsdfl_ctx* c, size_t P, size_t N)
     return TSDFL_OK;
 }
 
-// need: resample_workspace_bytes(M) or residual_workspace_bytes(M).
-int ensure_resample_ws(tsdfl_ctx* c, size_t need)
+// One size for the systematic and the residual systematic resampler: neither's call
+// moves the workspace under a graph captured from the other's.
+int ensure_resample_ws(tsdfl_ctx* c, size_t M)
 {
+    size_t need = std::max(resample_workspace_bytes(M), residual_workspace_bytes(M));
     if (need <= c->rs_bytes) return TSDFL_OK;
     need = std::max(need, c->rs_bytes + c->rs_bytes / 4);
     void* p = nullptr;
@@ -222,6 +226,27 @@ int ensure_resample_ws(tsdfl_ctx* c, size_t need)
     c->rs_ws = p;
     c->rs_bytes = need;
     return TSDFL_OK;
+}
+
+// The tables of the residual resampler's parallel form, or null where one thread walks
+// the chain: small clouds, and larger ones than the tables allow for when they cannot
+// grow (the stream is being captured, or the device is out of memory).
+void* residual_tables(tsdfl_ctx* c, size_t M)
+{
+    const size_t need = residual_tables_bytes(M);
+    if (need > c->rt_bytes) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        void* p = nullptr;
+        if (cudaStreamIsCapturing(c->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone ||
+            cudaMalloc(&p, std::max(need, c->rt_bytes + c->rt_bytes / 4)) != cudaSuccess) {
+            cudaGetLastError();   // not an error of the call
+            return nullptr;
+        }
+        if (c->rt_ws) cudaFree(c->rt_ws);
+        c->rt_ws = p;
+        c->rt_bytes = std::max(need, c->rt_bytes + c->rt_bytes / 4);
+    }
+    return need ? c->rt_ws : nullptr;
 }
 
 int ensure_scan_ws(tsdfl_ctx* c, size_t n)
@@ -785,6 +810,7 @@ int tsdfl_ctx_destroy(tsdfl_ctx* c)
     if (c->stream) cudaStreamSynchronize(c->stream);
     cudaFree(c->ws);
     cudaFree(c->rs_ws);
+    cudaFree(c->rt_ws);
     cudaFree(c->scan_ws);
     cudaFree(c->aux_ws);
     cudaFree(c->io);
@@ -840,7 +866,7 @@ int tsdfl_ctx_workspace_bytes(const tsdfl_ctx* c, size_t* eval_bytes, size_t* re
 {
     if (!c) return TSDFL_ERR_INVALID_ARG;
     if (eval_bytes) *eval_bytes = c->ws_bytes;
-    if (resample_bytes) *resample_bytes = c->rs_bytes;
+    if (resample_bytes) *resample_bytes = c->rs_bytes + c->rt_bytes;
     return TSDFL_OK;
 }
 
@@ -868,7 +894,10 @@ int tsdfl_ctx_reserve(tsdfl_ctx* c, size_t P, size_t N)
     if (rc) return rc;
     rc = ensure_workspace(c, P, N);
     if (rc) return rc;
-    return ensure_resample_ws(c, std::max(resample_workspace_bytes(P), residual_workspace_bytes(P)));
+    rc = ensure_resample_ws(c, P);
+    if (rc) return rc;
+    residual_tables(c, std::min(P, kMaxResidual - 1));   // without them its calls take longer
+    return TSDFL_OK;
 }
 
 int tsdfl_map_create(tsdfl_ctx* ctx, const tsdfl_map_coef* coef, const int32_t* grid_occ, const float* data,
@@ -1150,7 +1179,7 @@ int resample_systematic_host(tsdfl_ctx* c, const char* fn, const float* src, siz
     }
     int rc = set_device(c->device);
     if (rc) return rc;
-    rc = ensure_resample_ws(c, resample_workspace_bytes(M));
+    rc = ensure_resample_ws(c, M);
     if (rc) return rc;
     size_t w_b = align_up(sizeof(float) * stride * M, 256);
     size_t i_b = align_up(sizeof(uint32_t) * (cap ? cap : 1), 256);
@@ -1199,7 +1228,7 @@ int tsdfl_resample_systematic_device(tsdfl_ctx* c, const float* d_particles, siz
     }
     int rc = set_device(c->device);
     if (rc) return rc;
-    rc = ensure_resample_ws(c, resample_workspace_bytes(M));
+    rc = ensure_resample_ws(c, M);
     if (rc) return rc;
     return launch_resample_impl(d_particles, d_particles + 6, 7, M, u0, d_particles_out, nullptr, cap, d_count,
                                 c->rs_ws, c->done, c->status, c->stream);
@@ -1214,13 +1243,13 @@ int tsdfl_resample_residual_systematic(tsdfl_ctx* c, const float* weights, size_
     }
     *count_out = 0;
     if (M == 0) return TSDFL_OK;
-    if (M >= (1ull << 24)) {
+    if (M >= kMaxResidual) {
         set_error("tsdfl_resample_residual_systematic: at most 2^24-1 particles");
         return TSDFL_ERR_UNSUPPORTED;
     }
     int rc = set_device(c->device);
     if (rc) return rc;
-    rc = ensure_resample_ws(c, residual_workspace_bytes(M));
+    rc = ensure_resample_ws(c, M);
     if (rc) return rc;
     size_t w_b = align_up(sizeof(float) * M, 256);
     size_t i_b = align_up(sizeof(uint32_t) * (cap ? cap : 1), 256);
@@ -1232,7 +1261,8 @@ int tsdfl_resample_residual_systematic(tsdfl_ctx* c, const float* weights, size_
     uint32_t* d_cnt = reinterpret_cast<uint32_t*>(io + w_b + i_b);
     cudaStream_t s = c->stream;
     CUDA_TRY(cudaMemcpyAsync(d_w, weights, sizeof(float) * M, cudaMemcpyHostToDevice, s));
-    rc = launch_resample_residual(nullptr, d_w, 1, M, u0, nullptr, d_idx, cap, d_cnt, c->rs_ws, c->status, s);
+    rc = launch_resample_residual(nullptr, d_w, 1, M, u0, nullptr, d_idx, cap, d_cnt, c->rs_ws,
+                                  residual_tables(c, M), c->status, s);
     if (rc) return rc;
     CUDA_TRY(cudaMemcpyAsync(c->h_count, d_cnt, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     if (cap) CUDA_TRY(cudaMemcpyAsync(idx_out, d_idx, sizeof(uint32_t) * cap, cudaMemcpyDeviceToHost, s));
@@ -1251,16 +1281,16 @@ int tsdfl_resample_residual_systematic_device(tsdfl_ctx* c, const float* d_parti
         return TSDFL_ERR_INVALID_ARG;
     }
     if (M == 0) return TSDFL_OK;
-    if (M >= (1ull << 24)) {
+    if (M >= kMaxResidual) {
         set_error("tsdfl_resample_residual_systematic_device: at most 2^24-1 particles");
         return TSDFL_ERR_UNSUPPORTED;
     }
     int rc = set_device(c->device);
     if (rc) return rc;
-    rc = ensure_resample_ws(c, residual_workspace_bytes(M));
+    rc = ensure_resample_ws(c, M);
     if (rc) return rc;
     return launch_resample_residual(d_particles, d_particles + 6, 7, M, u0, d_particles_out, nullptr, cap, d_count,
-                                    c->rs_ws, c->status, c->stream);
+                                    c->rs_ws, residual_tables(c, M), c->status, c->stream);
 }
 
 int tsdfl_best_particle_device(tsdfl_ctx* c, const float* d_particles, size_t M, uint32_t* d_index)

@@ -754,52 +754,70 @@ int window_of(size_t M)
 
 size_t up(size_t v) { return (v + 255) / 256 * 256; }
 
-size_t layout(size_t M, char* p, ResidualWs* ws)
-{
-    const int tile = tile_of(M), window = window_of(M);
-    const size_t S = (M + tile - 1) / tile;
-    const bool par = M >= kParallelFrom;
+// The one-thread walk's part and the parallel form's tables, each in a buffer of its own.
+struct Carve {
+    char* p;
     size_t at = 0;
-    auto take = [&](size_t bytes) {
-        const size_t o = at;
-        at += up(bytes);
-        return p ? p + o : nullptr;
-    };
-    ResidualWs r{};
-    r.S = (int)S;
-    r.tile = tile;
-    r.window = window;
-    r.total = reinterpret_cast<unsigned long long*>(take(8));
-    r.err = reinterpret_cast<int*>(take(4));
-    r.mode = reinterpret_cast<int*>(take(4));
-    r.cnt = reinterpret_cast<uint32_t*>(take(4 * M));
-    r.off = reinterpret_cast<uint32_t*>(take(4 * M));
-    if (par) {
-        r.tiles = reinterpret_cast<TileSums*>(take(sizeof(TileSums) * S));
-        r.segs = reinterpret_cast<Seg*>(take(sizeof(Seg) * (S + 1)));
-        r.sums = reinterpret_cast<double*>(take(8 * S));
-        r.start = reinterpret_cast<float*>(take(4 * (S + 1)));
-        r.base = reinterpret_cast<uint32_t*>(take(4 * (S + 1)));
-        r.table = reinterpret_cast<uint32_t*>(take(4 * S * (size_t)window));
+    template <typename T>
+    T* take(size_t n)
+    {
+        T* r = p ? reinterpret_cast<T*>(p + at) : nullptr;
+        at += up(sizeof(T) * n);
+        return r;
     }
-    if (ws) *ws = r;
-    return at;
+};
+
+size_t layout_walk(size_t M, void* p, ResidualWs* ws)
+{
+    Carve a{static_cast<char*>(p)};
+    ws->total = a.take<unsigned long long>(1);
+    ws->err = a.take<int>(1);
+    ws->mode = a.take<int>(1);
+    ws->cnt = a.take<uint32_t>(M);
+    ws->off = a.take<uint32_t>(M);
+    return a.at;
+}
+
+size_t layout_tables(size_t M, void* p, ResidualWs* ws)
+{
+    Carve a{static_cast<char*>(p)};
+    ws->tile = tile_of(M);
+    ws->window = window_of(M);
+    ws->S = (int)((M + (size_t)ws->tile - 1) / (size_t)ws->tile);
+    const size_t S = (size_t)ws->S;
+    ws->tiles = a.take<TileSums>(S);
+    ws->segs = a.take<Seg>(S + 1);
+    ws->sums = a.take<double>(S);
+    ws->start = a.take<float>(S + 1);
+    ws->base = a.take<uint32_t>(S + 1);
+    ws->table = a.take<uint32_t>(S * (size_t)ws->window);
+    return a.at;
 }
 
 }  // namespace
 
-size_t residual_workspace_bytes(size_t M) { return layout(M ? M : 1, nullptr, nullptr); }
+size_t residual_workspace_bytes(size_t M)
+{
+    ResidualWs ws{};
+    return layout_walk(M, nullptr, &ws);
+}
+
+size_t residual_tables_bytes(size_t M)
+{
+    ResidualWs ws{};
+    return M < kParallelFrom ? 0 : layout_tables(M, nullptr, &ws);
+}
 
 int launch_resample_residual(const float* particles, const float* w, int stride, size_t M, float u0, float* out,
-                             uint32_t* idx_out, size_t cap, uint32_t* count_out, void* workspace, int32_t* status,
-                             cudaStream_t s)
+                             uint32_t* idx_out, size_t cap, uint32_t* count_out, void* workspace, void* tables,
+                             int32_t* status, cudaStream_t s)
 {
-    ResidualWs ws;
-    layout(M, static_cast<char*>(workspace), &ws);
+    ResidualWs ws{};
+    layout_walk(M, workspace, &ws);
     const int m = (int)M;
     const long long c = (long long)cap;
     // a draw outside [0, 1) is walked literally
-    if (M < kParallelFrom || !(u0 >= 0.0f) || !(u0 < 1.0f)) {
+    if (M < kParallelFrom || !tables || !(u0 >= 0.0f) || !(u0 < 1.0f)) {
         cudaError_t e = launch_chained(residual_chain_kernel, 1, kChainThreads, 0, s, w, stride, m, u0, ws.cnt, ws.off,
                                        ws.total, ws.err);
         if (e == cudaSuccess)
@@ -811,6 +829,7 @@ int launch_resample_residual(const float* particles, const float* w, int stride,
         const cudaError_t last = cudaGetLastError();
         return check(e == cudaSuccess ? last : e);
     }
+    layout_tables(M, tables, &ws);
     const size_t seg_smem = sizeof(float) * ((size_t)ws.tile + kHead + 4);
     const size_t follow_fixed = sizeof(Seg) * (ws.S + 1) + 4 * (((size_t)ws.S + 1 + 3) / 4 * 4);
     const size_t follow_smem = std::min(kFollowSmem, follow_fixed + 4 * (size_t)ws.S * ws.window);

@@ -342,11 +342,15 @@ size_t resample_workspace_bytes(size_t M);
 int launch_resample_impl(const float* particles, const float* w, int stride, size_t M, float u0, float* out,
                          uint32_t* idx_out, size_t cap, uint32_t* count_out, void* workspace, uint32_t* done,
                          int32_t* status, cudaStream_t s, const float* u0p = nullptr);
-// ResidualSystematicResampler on the device (residual.cu); workspace: residual_workspace_bytes(M).
+// ResidualSystematicResampler on the device (residual.cu); workspace: residual_workspace_bytes(M);
+// tables: residual_tables_bytes(M) (0 for small clouds), or null: one thread then walks
+// the chain, to the same results.  M below kMaxResidual.
+constexpr size_t kMaxResidual = size_t(1) << 24;
 size_t residual_workspace_bytes(size_t M);
+size_t residual_tables_bytes(size_t M);
 int launch_resample_residual(const float* particles, const float* w, int stride, size_t M, float u0, float* out,
-                             uint32_t* idx_out, size_t cap, uint32_t* count_out, void* workspace, int32_t* status,
-                             cudaStream_t s);
+                             uint32_t* idx_out, size_t cap, uint32_t* count_out, void* workspace, void* tables,
+                             int32_t* status, cudaStream_t s);
 int launch_best_particle(const float* particles, size_t M, unsigned long long* key, uint32_t* index_out, int sm_count,
                          cudaStream_t s);
 int launch_codes_from_floats(const float* data, size_t n, const float* code_values, float init_value,
