@@ -106,6 +106,7 @@ struct tsdfl_map {
     uint32_t hash_slots = 0, hash_probes = 0;
     float* values = nullptr;      // kNumCodes likelihood values (device)
     float max_value = 0;
+    bool finite = true;           // every likelihood value
     uint64_t bricks = 0;
     uint64_t bytes = 0;
 };
@@ -631,7 +632,10 @@ int map_common(tsdfl_ctx* ctx, const tsdfl_map_coef* coef, const int32_t* grid_o
     float vals[kNumCodes];
     code_values(sigma, coef->init_value, vals);
     m->max_value = 0;
-    for (int k = 0; k < kNumCodes; ++k) m->max_value = std::fmax(m->max_value, std::fabs(vals[k]));
+    for (int k = 0; k < kNumCodes; ++k) {
+        m->max_value = std::fmax(m->max_value, std::fabs(vals[k]));
+        m->finite = m->finite && std::isfinite(vals[k]);
+    }
     CUDA_TRY(cudaMalloc(&m->values, sizeof(vals)));
     CUDA_TRY(cudaMemcpyAsync(m->values, vals, sizeof(vals), cudaMemcpyHostToDevice, ctx->stream));
     // -1 beyond the table, up to every brick index a lookup inside the tiled
@@ -653,6 +657,10 @@ int map_common(tsdfl_ctx* ctx, const tsdfl_map_coef* coef, const int32_t* grid_o
     return TSDFL_OK;
 }
 
+// Whether the tiled kernels sum this map's values and the hits in one word.  The
+// fixed-point forms of infinities and NaN reach into the hits' bits.
+int packed_sums(const tsdfl_map* m, int shift) { return m->finite && packs(m->max_value, shift) ? 1 : 0; }
+
 int run_eval(tsdfl_ctx* c, const tsdfl_map* map, const tsdfl_model* mdl, float* d_particles, size_t P,
              const float* d_points, size_t N, const float tf[16], uint32_t flags, float* d_pose, uint32_t* d_dbg)
 {
@@ -671,7 +679,7 @@ int run_eval(tsdfl_ctx* c, const tsdfl_map* map, const tsdfl_model* mdl, float* 
     const float c_in = mdl->a_range * inv_max_range;
     const float c_out = mdl->a_max;
     const int shift = fixed_shift(map->max_value, (double)N);
-    b.packed = packs(map->max_value, shift);
+    b.packed = packed_sums(map, shift);
     const int npad = (int)align_up(N, 4);
     cudaStream_t s = c->stream;
     const bool order = order_particles(P, N);
@@ -727,7 +735,7 @@ int run_eval_sub(tsdfl_ctx* c, const tsdfl_map* map, const tsdfl_model* mdl, flo
     const float c_in = mdl->a_range * inv_max_range;
     const float c_out = mdl->a_max;
     const int shift = fixed_shift(map->max_value, (double)K);
-    b.packed = packs(map->max_value, shift);
+    b.packed = packed_sums(map, shift);
     const int npad = (int)align_up(N, 4);
     cudaStream_t s = c->stream;
     const bool order = order_particles(P, K, kOrderFromSub);
@@ -1495,7 +1503,7 @@ void per_configure(tsdfl_batch::Per& q, const tsdfl_filter& F, int sm_count)
     q.b.particles = F.d_particles;
     q.npad = (int)align_up(F.N, 4);
     q.shift = fixed_shift(F.map->max_value, (double)F.N);
-    q.b.packed = packs(F.map->max_value, q.shift);
+    q.b.packed = packed_sums(F.map, q.shift);
     const MapView& m = F.map->view;
     q.dense = F.map->occ != nullptr;
     q.tiled = m.storage == 0 && m.tiled != 0;
