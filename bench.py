@@ -76,7 +76,7 @@ def make_workload(args):
 # profiles/eval_tiled_kernel_building_20k_x_8192.md and
 # profiles/eval_tiled_kernel_global_1m_x_2048.md)
 MEASURED_TRAFFIC = {("building", 100_000, 8192, "compact", "fast"): 1.148179e9 + 0.008796e9,
-                    ("global", 1_000_000, 2048, "compact", "fast"): 26.0e9}
+                    ("global", 1_000_000, 2048, "compact", "fast"): 29.35e9 + 0.270690e9}
 
 
 def roofline_bytes(P: int, N: int, layout: str) -> float:
@@ -1005,9 +1005,11 @@ def main():
     achieved = alg / (kmed / 1000.0) / 1e9
     measured_traffic = MEASURED_TRAFFIC
     traffic = measured_traffic.get((args.workload, P, Npts, args.layout, args.kernel))
+    kernel = "eval_spread_kernel" if args.workload == "global" else "eval_tiled_kernel"
+    if args.kernel != "fast" or not info["fast_index"]:
+        kernel = "eval_exact_kernel"
     roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-            "traffic": traffic, "kernel": "eval_tiled_kernel" if (args.kernel == "fast" and info["fast_index"])
-            else "eval_exact_kernel", "kernel_ms": kmed, "peak_source": peak_src,
+            "traffic": traffic, "kernel": kernel, "kernel_ms": kmed, "peak_source": peak_src,
             "algorithmic_bytes": alg,
             "traffic_gbs": traffic / (kmed / 1000.0) / 1e9 if traffic else None}
 

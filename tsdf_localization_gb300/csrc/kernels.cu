@@ -914,7 +914,10 @@ constexpr int kSpreadWarps = kSpreadThreads / 32;
 // with a bitmap in shared memory their rings leave the L1 too little for the codes
 // of neighbouring particles (150,000 x 200 of 4,096 points, warehouse, us: brick table
 // 338 with 1,024 threads, 394 with 768, compact layout 515 and 427; 150,000 x 200 of 2,048,
-// building, compact: 374 to 464 from one process to the next, and 416).
+// building, compact: 374 to 464 from one process to the next, and 416).  The layout
+// decides the form too, which is not always the faster: every map has the brick
+// table, and through it (1,024 threads, the scan in shared memory) 300,000 x 256 of
+// 2,048 points on the compact building take 732 us, through the bitmap 791.
 __host__ __device__ constexpr int sub_threads(bool dense) { return dense ? 768 : 1024; }
 constexpr int kRing = 64;   // deferred lookups per warp (transformed point + scan index)
 constexpr uint32_t kDbgSlow = 0x10000u;   // debug code flag: decided by the exact slow tiers
@@ -1006,8 +1009,8 @@ struct TiledParams {
 // DBG: per-point codes are written to the debug buffer; MIN0: the map's min
 // corner is the origin, so offsets are the transformed coordinates.
 // LONG: chunk_pts may exceed 64 kPackedSteps (the batch kernel's, whose steps
-// stay single: in pairs 3.61 against 3.58 ms for 24 filters); otherwise two steps'
-// gathers are in flight at a time.
+// stay single: in pairs 24 filters take 1.71 ms an update, singly 1.73); otherwise
+// two steps' gathers are in flight at a time.
 // PACKED: values and hits in one word (LutEntry).
 template <int LAY, bool TWO, bool DBG, bool MIN0, bool LONG, bool PACKED>
 __device__ __forceinline__ void tiled_item(const EvalParams& p, const MapView& m, const MapView* s_map,
@@ -1220,6 +1223,8 @@ __global__ void __launch_bounds__(kTiledThreads, 1) eval_tiled_kernel(TiledParam
 
 constexpr int kSpreadBlocks = 2;      // 64-point blocks of the scan a work item holds in registers
 constexpr int kSpreadGroup = 16;      // particles a work item scores against them
+// a lane's packed sum of 2 kSpreadBlocks lookups, kPackedLookups of which stay below 2^56
+static_assert((2ull * kSpreadBlocks << 29) / kPackedLookups < 1ull << 25, "eval_spread_kernel's parts of a sum");
 constexpr int kRegionGroups = 1024;   // groups of neighbouring particles a region (512: 9.4, 2,048: 9.3, 8,192: 9.6 ms)
 
 struct SpreadParams {
@@ -1259,7 +1264,7 @@ __device__ __noinline__ void drain_to_particles(const MapView* m, const LutEntry
 // once an item: no pass is staged, one launch covers any scan.
 // One million particles x 2,048 points in the building: 1,024-point chunks of
 // points in shared memory, dealt out in advance, 12.7 ms and 63 GB of DRAM; the
-// same taken from a counter 10.9 ms and 49 GB; this walk 9.1 ms and 26 GB (2.9
+// same taken from a counter 10.9 ms and 49 GB; this walk 9.2 ms and 29 GB (3.2
 // TB/s).  It waits on its gathers now (issue 47 %, L1 tags 48 %): 640 threads of
 // 96 registers 9.1 ms, 768 of 80 9.6; two particles' gathers in flight a warp
 // 10.4, four blocks of points an item 10.6, one 10.2.
@@ -1439,8 +1444,9 @@ size_t spread_smem_bytes(uint32_t occ_bytes)
 // range term), written directly (one warp owns the particle).
 // Waits on the codes' gathers.  300,000 particles x 256 of 2,048 points in the
 // 100 x 100 m building, compact layout, a pass: 1,018 us with two 64-bit divisions a
-// point for its stratum and particles dealt to the warps in turn; 815 with the
-// strata stepped and particles from a counter.  STAGED: the scan in shared memory,
+// point for its stratum and particles dealt to the warps in turn; 791 with the
+// strata stepped and particles from a counter (704 with 1,024 threads
+// and the scan beside the bitmap, which larger scans lose more by: sub_threads).  STAGED: the scan in shared memory,
 // one 16-byte read a point instead of four from the SoA arrays.
 struct SubParams {
     EvalParams e;
@@ -1589,7 +1595,7 @@ __global__ void __launch_bounds__(sub_threads(DENSE), 1) eval_subsample_kernel(S
 }
 
 // Work items per batch, the unit in which the persistent multi-filter launch's
-// work is reported and its grid is bounded.
+// work is reported (tsdfl_batch_info).
 constexpr int kBatchItems = kTiledWarps * 8;
 
 struct BatchSeg {
@@ -1746,6 +1752,7 @@ __global__ void __launch_bounds__(256) eval_serial_kernel(EvalParams p)
 constexpr int kNormBlocks = 256;
 constexpr int kNormThreads = 256;
 constexpr int kNormSums = 10;
+constexpr int kNormalizeBlocks = 4 * 148;   // most blocks of normalize_kernel beside its first: about four an SM
 
 struct NormParams {
     int P;
@@ -3272,7 +3279,7 @@ int launch_eval_subsample(const MapView& m, float a_hit, int P, int N, int K, un
     const int need = (P + warps_cta - 1) / warps_cta;
     if (need < blocks) blocks = need > 0 ? need : 1;
     sp.work = b.work;
-    sp.group = P >= 32 * blocks * warps_cta ? 2 : 1;   // 300,000 x 256 (1,024 threads): 711 us, 718 singly, 732 in fours
+    sp.group = P >= 32 * blocks * warps_cta ? 2 : 1;   // 300,000 x 256, building, compact: 791 us, 806 singly, 800 in fours
     sp.items = (P + sp.group - 1) / sp.group;
     k<<<blocks, threads, smem, s>>>(sp);
     g_launches += 1;
@@ -3386,7 +3393,7 @@ int launch_norm(int P, int mode, int shift, double a_hit, double c_in, double c_
         g_launches += 5;
     } else {
         // at most a few blocks an SM: each adds the weight sum's partials once
-        const unsigned blocks = (unsigned)std::min((P + kNormThreads - 1) / kNormThreads, 4 * 148);
+        const unsigned blocks = (unsigned)std::min((P + kNormThreads - 1) / kNormThreads, kNormalizeBlocks);
         launch_chained(normalize_kernel, 1u + blocks, kNormThreads, 0, s, P, b, particles_out, pose_out, nb, sticky);
         g_launches += 1;
     }
